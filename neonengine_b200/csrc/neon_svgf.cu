@@ -7,8 +7,12 @@
 // CPU restatement bit for bit.  No CPU fallback exists.
 //
 // Redesign relative to the shaders (results unchanged):
-//  * the moments image is double-buffered, so a pass never reads what it writes (the shaders update
-//    it in place while neighbours read it);
+//  * the moments image is held as two planes, {history length, second moment} and {first moment,
+//    variance}, each double-buffered, so a pass never reads what it writes (the shaders update the
+//    image in place while neighbours read it) and the filter moves only the plane it changes;
+//  * every filter pass reads one of the two history images, none reads the storage image: what all
+//    but the last pass write there is overwritten unseen, so only the last pass sums colours;
+//  * the temporal pass leaves {normal, depth} as one 16-byte vector per pixel for the filter's taps;
 //  * the copy of the storage image into the history image (the shaders' "iteration 98" dispatch) is
 //    done by the last filter pass itself whenever that pass does not read the image being replaced
 //    (always the case for an odd iteration count, the reference's 3);
@@ -33,25 +37,64 @@ __device__ __forceinline__ float max_glsl(float a, float b) { return a < b ? b :
 __device__ __forceinline__ float min_glsl(float a, float b) { return b < a ? b : a; }
 __device__ __forceinline__ float mixf(float x, float y, float a) { return x * (1.0f - a) + y * a; }
 
-// 2^x: nearest-integer split, degree-7 polynomial of 2^f on [-0.5, 0.5], exact scaling by 2^n.
-// Inside (-126, 128) the nearest integer (ties to even) comes from adding and subtracting 1.5 * 2^23,
-// whose sum also carries that integer in its low mantissa bits: two additions on the main pipes
-// instead of a rounding and a conversion instruction, same values.
-__device__ __forceinline__ float exp2_poly(float x) {
-    if (!(x > -126.0f && x < 128.0f)) return x != x ? x : (x > 0.0f ? INFINITY : 0.0f);
-    const float magic = 12582912.0f;
-    const float shifted = x + magic;
-    const float n = shifted - magic, f = x - n;
-    float p = 1.5252734e-5f;
-    p = fmaf(p, f, 1.5403530e-4f);
-    p = fmaf(p, f, 1.3333558e-3f);
-    p = fmaf(p, f, 9.6181291e-3f);
-    p = fmaf(p, f, 5.5504109e-2f);
-    p = fmaf(p, f, 2.4022651e-1f);
-    p = fmaf(p, f, 6.9314718e-1f);
-    p = fmaf(p, f, 1.0f);
-    // (n + 127) << 23 with n = bits(shifted) - bits(magic)
-    return p * __uint_as_float((__float_as_uint(shifted) - 0x4B400000u + 127u) << 23);
+// Two floats in one 64-bit register: one instruction works on both, each rounded as the scalar operation rounds it.
+// The assembler contracts a packed multiplication and the packed addition of its result into one fused operation, .rn
+// and -fmad=false notwithstanding; a product that is added is therefore formed as a fused multiply-add of -0 (the same
+// value, and nothing left to fuse), the -0 coming from a kernel argument so that it is not folded away.
+using F2 = unsigned long long;
+constexpr F2 kNegZero2 = 0x8000000080000000ull;
+__device__ __forceinline__ F2 pack2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(F2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// max_glsl(v, 0) up to the sign of a zero: a NaN stays a NaN
+__device__ __forceinline__ float max0_nan(float v) {
+    float r;
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// 2^x for two x <= 0 (or NaN): nearest-integer split, degree-7 polynomial of 2^f on [-0.5, 0.5], exact scaling by 2^n;
+// 0 for x <= -126.  The nearest integer (ties to even) comes from adding and subtracting 1.5 * 2^23, whose sum also
+// carries that integer in its low mantissa bits: two additions on the main pipes instead of a rounding and a
+// conversion instruction, same values.
+__device__ __forceinline__ F2 exp2_poly2(F2 x) {
+    const F2 shifted = add2(x, pack2(12582912.0f, 12582912.0f));
+    const F2 n = add2(shifted, pack2(-12582912.0f, -12582912.0f));
+    const F2 f = fma2(n, pack2(-1.0f, -1.0f), x);  // x - n: the product is exact
+    F2 p = pack2(1.5252734e-5f, 1.5252734e-5f);
+    p = fma2(p, f, pack2(1.5403530e-4f, 1.5403530e-4f));
+    p = fma2(p, f, pack2(1.3333558e-3f, 1.3333558e-3f));
+    p = fma2(p, f, pack2(9.6181291e-3f, 9.6181291e-3f));
+    p = fma2(p, f, pack2(5.5504109e-2f, 5.5504109e-2f));
+    p = fma2(p, f, pack2(2.4022651e-1f, 2.4022651e-1f));
+    p = fma2(p, f, pack2(6.9314718e-1f, 6.9314718e-1f));
+    p = fma2(p, f, pack2(1.0f, 1.0f));
+    float x0, x1, s0, s1;
+    unpack2(x, x0, x1);
+    unpack2(shifted, s0, s1);
+    // (n + 127) << 23 with n = bits(shifted) - bits(1.5 * 2^23), whose low nine bits are zero
+    const F2 scale = pack2(__uint_as_float((__float_as_uint(s0) << 23) + 0x3F800000u), __uint_as_float((__float_as_uint(s1) << 23) + 0x3F800000u));
+    float r0, r1;
+    unpack2(mul2(p, scale), r0, r1);
+    return pack2(x0 <= -126.0f ? 0.0f : r0, x1 <= -126.0f ? 0.0f : r1);
 }
 
 __device__ __forceinline__ unsigned to_unorm8(float v) {
@@ -83,9 +126,13 @@ struct Frame {  // the caller's images of one frame
 constexpr int kBlockX = 32, kBlockY = 8;
 
 // ---- temporal accumulation (raytracing_pp.comp:35-247, display mode 5) ---------------------------
+// a = {history length, second moment}, b = {first moment, variance}.  Also leaves what the filter passes read of the
+// G-buffer: guide = {normal, depth} and whether the pixel shows a surface.
 __global__ void __launch_bounds__(kBlockX* kBlockY) k_temporal(int w, int h, Frame fr, const uint2* __restrict__ hist_prev,
-                                                               uint2* __restrict__ hist_next, const float4* __restrict__ data_in,
-                                                               float4* __restrict__ data_out) {
+                                                               uint2* __restrict__ hist_next, const float2* __restrict__ a_in,
+                                                               const float2* __restrict__ b_in, float2* __restrict__ a_out,
+                                                               float2* __restrict__ b_out, float4* __restrict__ guide,
+                                                               uint8_t* __restrict__ surface) {
     const int x = blockIdx.x * kBlockX + threadIdx.x, y = blockIdx.y * kBlockY + threadIdx.y;
     if (x >= w || y >= h) return;
     const size_t idx = (size_t)y * w + x;
@@ -96,7 +143,8 @@ __global__ void __launch_bounds__(kBlockX* kBlockY) k_temporal(int w, int h, Fra
     float pr = 0.0f, pg = 0.0f, pb = 0.0f, hl = 0.0f, pm0 = 0.0f, pm1 = 0.0f;
     bool ok = false;
     const float4 cp = __ldg(fr.pos + idx), cn = __ldg(fr.nrm + idx);
-    if (!(dot3(cp.x, cp.y, cp.z, cp.x, cp.y, cp.z) < 1e-6f)) {
+    const bool none = dot3(cp.x, cp.y, cp.z, cp.x, cp.y, cp.z) < 1e-6f;
+    if (!none) {
         const float4 cbary = __ldg(fr.bary + idx), m = __ldg(fr.mot + idx);
         const int cur_mesh = (int)roundf(cn.w);
         const float uvx = ((float)x + 0.5f) / (float)w, uvy = ((float)y + 0.5f) / (float)h;
@@ -128,10 +176,10 @@ __global__ void __launch_bounds__(kBlockX* kBlockY) k_temporal(int w, int h, Fra
                 const float wt = weights[i];
                 const float3 hc = load_rgb16(hist_prev, t);
                 ar += hc.x * wt; ag += hc.y * wt; ab += hc.z * wt;
-                const float4 td = __ldg(data_in + t);
-                ah += td.x * wt;
-                am0 += td.y * wt;
-                am1 += td.z * wt;
+                const float2 ta = __ldg(a_in + t);
+                ah += ta.x * wt;
+                am0 += __ldg(&b_in[t].x) * wt;
+                am1 += ta.y * wt;
                 aw += wt;
             }
             if (!(aw < 0.5f)) {
@@ -161,70 +209,145 @@ __global__ void __launch_bounds__(kBlockX* kBlockY) k_temporal(int w, int h, Fra
     m1 = mixf(pm1, m1, alpha);
     const float variance = max_glsl(0.0f, m1 - m0 * m0);
     hist_next[idx] = pack_rgba16(nr, ng, nb, 1.0f);
-    data_out[idx] = make_float4(hl, m0, m1, variance);
-    fr.image[idx] = pack_rgb8(nr, ng, nb);
+    a_out[idx] = make_float2(hl, m1);
+    b_out[idx] = make_float2(m0, variance);
+    guide[idx] = make_float4(cn.x, cn.y, cn.z, cp.z);
+    surface[idx] = none ? 0 : 1;
 }
 
 // ---- a-trous filter pass (raytracing_atrous.comp:59-160, iteration < 98) -------------------------
-// copy_to != nullptr: the pass also stores its rgba8 result, converted back to floats, into that
+// One CTA filters a tile of 32 x 16 pixels from shared memory, where the tile and its halo of two steps on each side
+// lie with the image's edges already repeated; a thread filters two pixels eight rows apart, so that everything after
+// the differences of a tap is one packed instruction for both.  Bound by instruction issue and the multiply-add pipe (25
+// taps of about 40 instructions); a 1080p frame with 3 passes takes 334 us against 562 us with one pixel a thread,
+// separate taps of 44 bytes through L1 and colours summed in every pass.  STEP 0: any step, taps from global memory (steps
+// beyond 8, whose halo no longer fits).
+// LAST: also the colour sums, the storage image and (copy_to != nullptr) its conversion back to floats in that
 // history image (the shaders' separate copy dispatch, raytracing_atrous.comp:66-70).
-__global__ void __launch_bounds__(kBlockX* kBlockY) k_atrous(int w, int h, int step, Frame fr, const uint2* __restrict__ colour,
-                                                             const float4* __restrict__ data_in, float4* __restrict__ data_out,
-                                                             uint2* __restrict__ copy_to) {
-    const int x = blockIdx.x * kBlockX + threadIdx.x, y = blockIdx.y * kBlockY + threadIdx.y;
-    if (x >= w || y >= h) return;
-    const size_t idx = (size_t)y * w + x;
+constexpr int kTileX = 32, kTileY = 16, kFilterThreads = 256;
+constexpr size_t tile_bytes(int step, bool last) { return (size_t)(kTileX + 4 * step) * (kTileY + 4 * step) * (last ? 32 : 24); }
+
+template <int STEP, bool LAST>
+__global__ void __launch_bounds__(kFilterThreads, STEP ? 3 : 2)
+k_atrous(int w, int h, int any_step, const float4* __restrict__ guide, const uint8_t* __restrict__ surface, const float2* __restrict__ b_in,
+         float2* __restrict__ b_out, const uint2* __restrict__ colour, uchar4* __restrict__ image, uint2* __restrict__ copy_to, F2 neg_zero) {
+    constexpr int pitch = kTileX + 4 * STEP, rows = kTileY + 4 * STEP, cells = pitch * rows;
+    extern __shared__ __align__(16) unsigned char tile[];
+    float4* tg = reinterpret_cast<float4*>(tile);
+    float2* tb = reinterpret_cast<float2*>(tile + (size_t)cells * 16);
+    uint2* tc = reinterpret_cast<uint2*>(tile + (size_t)cells * 24);
+    const int tid = threadIdx.x, lx = tid & 31, ly = tid >> 5;
+    const int x0 = blockIdx.x * kTileX, y0 = blockIdx.y * kTileY;
+    const int step = STEP ? STEP : any_step;
+    if (STEP) {
+        for (int i = tid; i < cells; i += kFilterThreads) {
+            const int r = i / pitch, c = i - r * pitch;
+            const int qx = min(max(x0 + c - 2 * STEP, 0), w - 1), qy = min(max(y0 + r - 2 * STEP, 0), h - 1);
+            const size_t q = (size_t)qy * w + qx;
+            const unsigned s16 = (unsigned)__cvta_generic_to_shared(tg + i), s8 = (unsigned)__cvta_generic_to_shared(tb + i);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s16), "l"(guide + q) : "memory");
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s8), "l"(b_in + q) : "memory");
+            if (LAST) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(tc + i)), "l"(colour + q) : "memory");
+        }
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+    }
+    const int x = x0 + lx;
+    const int ya = y0 + ly, yb = ya + 8;
+    if (x >= w || ya >= h) return;
+    const bool have_b = yb < h;
+    const size_t ia = (size_t)ya * w + x, ib = have_b ? (size_t)yb * w + x : ia;
+    // tap (yy, xx) of the pixel `down` rows below this thread's first one
+    auto cell = [&](int yy, int xx, int down) -> size_t {
+        if (STEP) return (size_t)((ly + down + (yy + 2) * STEP) * pitch + lx + (xx + 2) * STEP);
+        // in 64 bits: rows * steps of a large image leave 32
+        const long long ty = (long long)(ya + down) + (long long)yy * step, tx = (long long)x + (long long)xx * step;
+        const int qy = (int)min(max(ty, 0ll), (long long)(h - 1)), qx = (int)min(max(tx, 0ll), (long long)(w - 1));
+        return (size_t)qy * w + qx;
+    };
+    const float4* gp = STEP ? tg : guide;
+    const float2* bp = STEP ? tb : b_in;
+    const uint2* cp = STEP ? tc : colour;
     const float eps = 1e-6f, log2e = 1.4426950408889634f, inv256 = 1.0f / 256.0f;
-    const float4 cp = __ldg(fr.pos + idx), cd = __ldg(data_in + idx);
-    uchar4 result;
-    float out_var = cd.w;
-    if (dot3(cp.x, cp.y, cp.z, cp.x, cp.y, cp.z) < eps) {  // no surface: the colour passes through
-        const float3 s = load_rgb16(colour, idx);
-        result = pack_rgb8(s.x, s.y, s.z);
-    } else {
-        const float4 cn = __ldg(fr.nrm + idx);
-        const float c_lum = cd.y, c_var = max_glsl(cd.w, 0.0f);
-        const float step_f = (float)step;
-        const float inv_z = 1.0f / max_glsl(fabsf(cp.z) * step_f, eps);
-        const float inv_l = 1.0f / max_glsl(1.0f * sqrtf(max_glsl(c_var, 1e-10f)), eps);
-        float sr = 0.0f, sg = 0.0f, sb = 0.0f, sum_w = 0.0f, sum_var = 0.0f, sum_wvar = 0.0f;
-#pragma unroll
+    const size_t ca = cell(0, 0, 0), cb = cell(0, 0, 8);
+    const float4 ga = gp[ca], gb = gp[cb];
+    const float2 ba = bp[ca], bb = bp[cb];
+    const float step_f = (float)step;
+    const float inv_za = 1.0f / max_glsl(fabsf(ga.w) * step_f, eps), inv_zb = 1.0f / max_glsl(fabsf(gb.w) * step_f, eps);
+    const float inv_la = 1.0f / max_glsl(1.0f * sqrtf(max_glsl(max_glsl(ba.y, 0.0f), 1e-10f)), eps);
+    const float inv_lb = 1.0f / max_glsl(1.0f * sqrtf(max_glsl(max_glsl(bb.y, 0.0f), 1e-10f)), eps);
+    const bool on_a = surface[ia] != 0, on_b = have_b && surface[ib] != 0;
+    F2 sum_r = 0, sum_g = 0, sum_b = 0, sum_w = 0, sum_var = 0, sum_wvar = 0;  // bits of two zeros
+    if (on_a || on_b) {
+        const F2 log2e2 = pack2(log2e, log2e);
+#pragma unroll 1
         for (int yy = -2; yy <= 2; ++yy) {
-            const int qy = min(max(y + yy * step, 0), h - 1);
             const float ky = yy == 0 ? 6.0f : ((yy == 1 || yy == -1) ? 4.0f : 1.0f);
 #pragma unroll
             for (int xx = -2; xx <= 2; ++xx) {
-                const int qx = min(max(x + xx * step, 0), w - 1);
                 const float kx = xx == 0 ? 6.0f : ((xx == 1 || xx == -1) ? 4.0f : 1.0f);
                 const float wk = kx * ky * inv256;
-                const size_t q = (size_t)qy * w + qx;
-                const float4 sn = __ldg(fr.nrm + q);
-                float wn = max_glsl(dot3(cn.x, cn.y, cn.z, sn.x, sn.y, sn.z), 0.0f);
-                wn *= wn; wn *= wn; wn *= wn; wn *= wn; wn *= wn; wn *= wn; wn *= wn;
-                if (wn <= eps) continue;
-                const float s_pos_z = __ldg(&fr.pos[q].z);
-                const float4 sd = __ldg(data_in + q);
-                const float3 sc = load_rgb16(colour, q);
-                const float s_var = max_glsl(sd.w, 0.0f);
-                const float dz = fabsf(cp.z - s_pos_z);
-                const float wd = exp2_poly(-dz * inv_z * log2e);
-                const float dl = fabsf(c_lum - sd.y);
-                const float wl = exp2_poly(-dl * inv_l * log2e);
-                const float wt = wk * wn * wd * wl;
-                sr += sc.x * wt; sg += sc.y * wt; sb += sc.z * wt;
-                sum_w += wt;
-                const float w2 = wt * wt;
-                sum_var += s_var * w2;
-                sum_wvar += w2;
+                const size_t qa = cell(yy, xx, 0), qb = cell(yy, xx, 8);
+                const float4 sa = gp[qa], sb = gp[qb];
+                const float2 va = bp[qa], vb = bp[qb];
+                F2 wn = pack2(max0_nan(dot3(ga.x, ga.y, ga.z, sa.x, sa.y, sa.z)), max0_nan(dot3(gb.x, gb.y, gb.z, sb.x, sb.y, sb.z)));
+#pragma unroll
+                for (int i = 0; i < 7; ++i) wn = mul2(wn, wn);
+                float wna, wnb;
+                unpack2(wn, wna, wnb);
+                const bool skip_a = wna <= eps, skip_b = wnb <= eps;  // such a tap adds nothing, whatever its values
+                const F2 wd = exp2_poly2(fma2(pack2(-fabsf(ga.w - sa.w) * inv_za, -fabsf(gb.w - sb.w) * inv_zb), log2e2, neg_zero));
+                const F2 wl = exp2_poly2(fma2(pack2(-fabsf(ba.x - va.x) * inv_la, -fabsf(bb.x - vb.x) * inv_lb), log2e2, neg_zero));
+                float wta, wtb;
+                unpack2(mul2(mul2(mul2(pack2(wk, wk), wn), wd), wl), wta, wtb);
+                const F2 wt = pack2(skip_a ? 0.0f : wta, skip_b ? 0.0f : wtb);
+                // variances are never negative (a NaN stays one), so the shader's max(variance, 0) changes nothing
+                const F2 sv = pack2(skip_a ? 0.0f : va.y, skip_b ? 0.0f : vb.y);
+                if (LAST) {
+                    uint2 pa = cp[qa], pb = cp[qb];
+                    if (skip_a) pa = make_uint2(0u, 0u);
+                    if (skip_b) pb = make_uint2(0u, 0u);
+                    const __half2 la = *reinterpret_cast<const __half2*>(&pa.x), lb = *reinterpret_cast<const __half2*>(&pb.x);
+                    const __half2 ha = *reinterpret_cast<const __half2*>(&pa.y), hb = *reinterpret_cast<const __half2*>(&pb.y);
+                    sum_r = add2(sum_r, fma2(pack2(__low2float(la), __low2float(lb)), wt, neg_zero));
+                    sum_g = add2(sum_g, fma2(pack2(__high2float(la), __high2float(lb)), wt, neg_zero));
+                    sum_b = add2(sum_b, fma2(pack2(__low2float(ha), __low2float(hb)), wt, neg_zero));
+                    sum_w = add2(sum_w, wt);
+                }
+                const F2 w2 = fma2(wt, wt, neg_zero);
+                sum_var = add2(sum_var, fma2(sv, w2, neg_zero));
+                sum_wvar = add2(sum_wvar, w2);
             }
         }
-        const float inv_w = 1.0f / max_glsl(sum_w, eps), inv_wv = 1.0f / max_glsl(sum_wvar, eps);
-        result = pack_rgb8(sr * inv_w, sg * inv_w, sb * inv_w);
-        out_var = sum_var * inv_wv;
     }
-    fr.image[idx] = result;
-    data_out[idx] = make_float4(cd.x, cd.y, cd.z, out_var);
-    if (copy_to) copy_to[idx] = pack_rgba16(result.x / 255.0f, result.y / 255.0f, result.z / 255.0f, result.w / 255.0f);
+    float sv[2], swv[2];
+    unpack2(sum_var, sv[0], sv[1]);
+    unpack2(sum_wvar, swv[0], swv[1]);
+    float sr[2], sg[2], sb[2], sw[2];
+    unpack2(sum_r, sr[0], sr[1]);
+    unpack2(sum_g, sg[0], sg[1]);
+    unpack2(sum_b, sb[0], sb[1]);
+    unpack2(sum_w, sw[0], sw[1]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if (k && !have_b) break;
+        const size_t idx = k ? ib : ia;
+        const float2 centre = k ? bb : ba;
+        const bool on = k ? on_b : on_a;  // no surface: colour and variance pass through
+        b_out[idx] = make_float2(centre.x, on ? sv[k] * (1.0f / max_glsl(swv[k], eps)) : centre.y);
+        if (LAST) {
+            uchar4 result;
+            if (on) {
+                const float inv_w = 1.0f / max_glsl(sw[k], eps);
+                result = pack_rgb8(sr[k] * inv_w, sg[k] * inv_w, sb[k] * inv_w);
+            } else {
+                const float3 s = load_rgb16(colour, idx);
+                result = pack_rgb8(s.x, s.y, s.z);
+            }
+            image[idx] = result;
+            if (copy_to) copy_to[idx] = pack_rgba16(result.x / 255.0f, result.y / 255.0f, result.z / 255.0f, result.w / 255.0f);
+        }
+    }
 }
 
 // ---- copy pass (raytracing_atrous.comp:66-70, iteration 98) ---------------------------------------
@@ -235,6 +358,20 @@ __global__ void k_copy(size_t n, const uchar4* __restrict__ image, uint2* __rest
     dst[i] = pack_rgba16(c.x / 255.0f, c.y / 255.0f, c.z / 255.0f, c.w / 255.0f);
 }
 
+// ---- the moments image {history length, first moment, second moment, variance} <-> its two planes ----
+__global__ void k_split_moments(size_t n, const float4* __restrict__ m, float2* __restrict__ a, float2* __restrict__ b) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 v = m[i];
+    a[i] = make_float2(v.x, v.z);
+    b[i] = make_float2(v.y, v.w);
+}
+__global__ void k_join_moments(size_t n, const float2* __restrict__ a, const float2* __restrict__ b, float4* __restrict__ m) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    m[i] = make_float4(a[i].x, b[i].x, a[i].y, b[i].y);
+}
+
 thread_local std::string g_svgf_create_error;
 
 }  // namespace
@@ -243,8 +380,11 @@ struct neon_svgf_handle {
     neon_svgf_config cfg{};
     std::string err;
     uint2 *colour_a = nullptr, *colour_b = nullptr;  // rgba16f history images
-    float4* data[2] = {nullptr, nullptr};            // moments: data[0] holds the state between frames
-    int ping_pong = 0;
+    float2* mom_a[2] = {nullptr, nullptr};           // {history length, second moment}: mom_a[cur_a] holds the state between frames
+    float2* mom_b[2] = {nullptr, nullptr};           // {first moment, variance}: mom_b[0] holds the state between frames
+    float4* guide = nullptr;                         // {normal, depth} of the frame being filtered
+    uint8_t* surface = nullptr;                      // whether its pixels show a surface
+    int ping_pong = 0, cur_a = 0;
     float4* stage[4] = {nullptr, nullptr, nullptr, nullptr};  // device copies of host G-buffers (denoise_host)
     uchar4* stage_image = nullptr;
     int64_t launches = 0;
@@ -253,7 +393,7 @@ struct neon_svgf_handle {
     cudaStream_t own_stream = nullptr, last_stream = nullptr;
     struct Cached {
         Frame fr;
-        int ping_pong;
+        int ping_pong, cur_a;
         cudaGraphExec_t exec;
     };
     std::vector<Cached> graphs;
@@ -283,21 +423,46 @@ void drop_graphs(neon_svgf_handle* h) {
     h->graphs.clear();
 }
 
+template <int STEP, bool LAST>
+void launch_atrous(neon_svgf_handle* h, int step, int from, const uint2* src, uchar4* image, uint2* copy_to, cudaStream_t st) {
+    const dim3 grid((h->cfg.width + kTileX - 1) / kTileX, (h->cfg.height + kTileY - 1) / kTileY);
+    k_atrous<STEP, LAST><<<grid, kFilterThreads, STEP ? tile_bytes(STEP, LAST) : 0, st>>>(
+        h->cfg.width, h->cfg.height, step, h->guide, h->surface, h->mom_b[from], h->mom_b[from ^ 1], src, image, copy_to, kNegZero2);
+}
+template <bool LAST>
+void launch_atrous(neon_svgf_handle* h, int step, int from, const uint2* src, uchar4* image, uint2* copy_to, cudaStream_t st) {
+    switch (step) {
+        case 1: launch_atrous<1, LAST>(h, step, from, src, image, copy_to, st); break;
+        case 2: launch_atrous<2, LAST>(h, step, from, src, image, copy_to, st); break;
+        case 4: launch_atrous<4, LAST>(h, step, from, src, image, copy_to, st); break;
+        case 8: launch_atrous<8, LAST>(h, step, from, src, image, copy_to, st); break;
+        default: launch_atrous<0, LAST>(h, step, from, src, image, copy_to, st);
+    }
+}
+// tiles above 48 KB of shared memory have to be asked for
+template <int STEP>
+bool allow_tile() {
+    return cudaFuncSetAttribute(k_atrous<STEP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes(STEP, false)) == cudaSuccess &&
+           cudaFuncSetAttribute(k_atrous<STEP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes(STEP, true)) == cudaSuccess;
+}
+
 // the kernels of one frame in the reference's dispatch order; ev (optional) gets 3 event marks.
-// ping_pong is the flag's value BEFORE the frame (RayTracingRast::renderCompute flips it).
-int record_frame(neon_svgf_handle* h, const Frame& fr, int ping_pong, cudaStream_t st, cudaEvent_t* ev = nullptr) {
+// ping_pong is the flag's value BEFORE the frame (RayTracingRast::renderCompute flips it), cur_a that of h->cur_a.
+int record_frame(neon_svgf_handle* h, const Frame& fr, int ping_pong, int cur_a, cudaStream_t st, cudaEvent_t* ev = nullptr) {
     const int w = h->cfg.width, ht = h->cfg.height, iters = h->cfg.atrous_iterations;
     const dim3 grid((w + kBlockX - 1) / kBlockX, (ht + kBlockY - 1) / kBlockY), block(kBlockX, kBlockY);
     // set 1 binds {5: colour_a, 7: colour_b}, set 2 the two swapped; the temporal pass takes set 1 when the flag is set
     uint2* prev = ping_pong ? h->colour_a : h->colour_b;
     uint2* next = ping_pong ? h->colour_b : h->colour_a;
-    int n = 0, cur = 0;  // data[cur] is read, data[cur ^ 1] written
+    int n = 0, cur = 0;  // mom_b[cur] is read, mom_b[cur ^ 1] written
     if (ev) cudaEventRecord(ev[0], st);
-    k_temporal<<<grid, block, 0, st>>>(w, ht, fr, prev, next, h->data[cur], h->data[cur ^ 1]); ++n;
+    k_temporal<<<grid, block, 0, st>>>(w, ht, fr, prev, next, h->mom_a[cur_a], h->mom_b[0], h->mom_a[cur_a ^ 1], h->mom_b[1], h->guide,
+                                       h->surface); ++n;
     cur ^= 1;
     if (ev) cudaEventRecord(ev[1], st);
     // filter passes: even ones read the image the temporal pass wrote, odd ones the older one; the
-    // even-count extra pass runs on the second set at step 1 (raytracing_rast.cpp:390-411)
+    // even-count extra pass runs on the second set at step 1 (raytracing_rast.cpp:390-411).  Their number
+    // is odd, so the variances end in mom_b[0].
     const int passes = iters + (iters % 2 == 0 ? 1 : 0);
     bool copied = false;
     for (int i = 0; i < passes; ++i) {
@@ -305,17 +470,16 @@ int record_frame(neon_svgf_handle* h, const Frame& fr, int ping_pong, cudaStream
         const uint2* src = extra ? prev : ((i % 2 == 0) ? next : prev);
         const bool last = i == passes - 1;
         uint2* copy_to = (last && src != prev) ? prev : nullptr;
-        k_atrous<<<grid, block, 0, st>>>(w, ht, extra ? 1 : (1 << i), fr, src, h->data[cur], h->data[cur ^ 1], copy_to); ++n;
+        const int step = extra ? 1 : (1 << i);
+        if (last) launch_atrous<true>(h, step, cur, src, fr.image, copy_to, st);
+        else launch_atrous<false>(h, step, cur, src, nullptr, nullptr, st);
+        ++n;
         cur ^= 1;
         copied = copy_to != nullptr;
     }
     if (!copied) {
         const size_t px = (size_t)w * ht;
         k_copy<<<(unsigned)((px + 255) / 256), 256, 0, st>>>(px, fr.image, prev); ++n;
-    }
-    if (cur != 0) {  // an odd number of passes: bring the moments back to data[0]
-        if (cudaMemcpyAsync(h->data[0], h->data[1], (size_t)w * ht * sizeof(float4), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-            return -1;
     }
     if (ev) cudaEventRecord(ev[2], st);
     h->launches_per_frame = n;
@@ -348,11 +512,13 @@ int neon_svgf_create(const neon_svgf_config* cfg, neon_svgf_handle** out) {
     h->cfg = *cfg;
     const size_t px = (size_t)cfg->width * cfg->height;
     bool ok = cudaSetDevice(cfg->device) == cudaSuccess && cudaMalloc(&h->colour_a, px * 8) == cudaSuccess &&
-              cudaMalloc(&h->colour_b, px * 8) == cudaSuccess && cudaMalloc(&h->data[0], px * 16) == cudaSuccess &&
-              cudaMalloc(&h->data[1], px * 16) == cudaSuccess &&
+              cudaMalloc(&h->colour_b, px * 8) == cudaSuccess && cudaMalloc(&h->guide, px * 16) == cudaSuccess &&
+              cudaMalloc(&h->surface, px) == cudaSuccess && allow_tile<4>() && allow_tile<8>() &&
               cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking) == cudaSuccess;
-    ok = ok && cudaMemset(h->colour_a, 0, px * 8) == cudaSuccess && cudaMemset(h->colour_b, 0, px * 8) == cudaSuccess &&
-         cudaMemset(h->data[0], 0, px * 16) == cudaSuccess && cudaMemset(h->data[1], 0, px * 16) == cudaSuccess;
+    ok = ok && cudaMemset(h->colour_a, 0, px * 8) == cudaSuccess && cudaMemset(h->colour_b, 0, px * 8) == cudaSuccess;
+    for (int i = 0; i < 2; ++i)
+        for (float2** m : {&h->mom_a[i], &h->mom_b[i]})
+            ok = ok && cudaMalloc(m, px * 8) == cudaSuccess && cudaMemset(*m, 0, px * 8) == cudaSuccess;
     if (!ok) {
         const cudaError_t e = cudaGetLastError();
         neon_svgf_destroy(h);
@@ -367,7 +533,8 @@ int neon_svgf_destroy(neon_svgf_handle* h) {
     cudaSetDevice(h->cfg.device);
     if (h->last_stream) cudaStreamSynchronize(h->last_stream);
     drop_graphs(h);
-    cudaFree(h->colour_a); cudaFree(h->colour_b); cudaFree(h->data[0]); cudaFree(h->data[1]);
+    cudaFree(h->colour_a); cudaFree(h->colour_b); cudaFree(h->guide); cudaFree(h->surface);
+    for (int i = 0; i < 2; ++i) { cudaFree(h->mom_a[i]); cudaFree(h->mom_b[i]); }
     for (auto* p : h->stage) cudaFree(p);
     cudaFree(h->stage_image);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
@@ -387,7 +554,21 @@ int neon_svgf_set_history(neon_svgf_handle* h, const uint16_t* colour_a, const u
     const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     if (colour_a) SCU(h, cudaMemcpy(h->colour_a, colour_a, px * 8, kind)); else SCU(h, cudaMemset(h->colour_a, 0, px * 8));
     if (colour_b) SCU(h, cudaMemcpy(h->colour_b, colour_b, px * 8, kind)); else SCU(h, cudaMemset(h->colour_b, 0, px * 8));
-    if (moments) SCU(h, cudaMemcpy(h->data[0], moments, px * 16, kind)); else SCU(h, cudaMemset(h->data[0], 0, px * 16));
+    h->cur_a = 0;
+    if (moments) {
+        float4* tmp = nullptr;
+        SCU(h, cudaMalloc(&tmp, px * 16));
+        cudaError_t e = cudaMemcpy(tmp, moments, px * 16, kind);
+        if (e == cudaSuccess) {
+            k_split_moments<<<(unsigned)((px + 255) / 256), 256, 0, h->own_stream>>>(px, tmp, h->mom_a[0], h->mom_b[0]);
+            e = cudaStreamSynchronize(h->own_stream);
+        }
+        cudaFree(tmp);
+        if (e != cudaSuccess) return sfail(h, NEON_MOE_ECUDA, "loading the moments failed: %s", cudaGetErrorString(e));
+    } else {
+        SCU(h, cudaMemset(h->mom_a[0], 0, px * 8));
+        SCU(h, cudaMemset(h->mom_b[0], 0, px * 8));
+    }
     h->ping_pong = ping_pong != 0;
     return NEON_MOE_OK;
 }
@@ -401,7 +582,7 @@ int neon_svgf_denoise(neon_svgf_handle* h, const float* position, const float* n
     const Frame fr{reinterpret_cast<const float4*>(position), reinterpret_cast<const float4*>(normal),
                    reinterpret_cast<const float4*>(barycentric), reinterpret_cast<const float4*>(motion),
                    reinterpret_cast<uchar4*>(image)};
-    const int pp = h->ping_pong;
+    const int pp = h->ping_pong, ca = h->cur_a;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     bool graphs = h->use_graphs != 0;
     if (graphs && (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) {
@@ -411,11 +592,11 @@ int neon_svgf_denoise(neon_svgf_handle* h, const float* position, const float* n
     if (graphs) {
         neon_svgf_handle::Cached* hit = nullptr;
         for (auto& g : h->graphs)
-            if (g.ping_pong == pp && !memcmp(&g.fr, &fr, sizeof fr)) { hit = &g; break; }
+            if (g.ping_pong == pp && g.cur_a == ca && !memcmp(&g.fr, &fr, sizeof fr)) { hit = &g; break; }
         if (!hit) {
             if (h->graphs.size() >= 32) drop_graphs(h);
             SCU(h, cudaStreamBeginCapture(h->own_stream, cudaStreamCaptureModeThreadLocal));
-            const int n = record_frame(h, fr, pp, h->own_stream);
+            const int n = record_frame(h, fr, pp, ca, h->own_stream);
             cudaGraph_t graph = nullptr;
             cudaError_t ce = cudaStreamEndCapture(h->own_stream, &graph);
             cudaGraphExec_t exec = nullptr;
@@ -426,7 +607,7 @@ int neon_svgf_denoise(neon_svgf_handle* h, const float* position, const float* n
                 h->use_graphs = 0;  // capture is not available here: stay eager
                 graphs = false;
             } else {
-                h->graphs.push_back({fr, pp, exec});
+                h->graphs.push_back({fr, pp, ca, exec});
                 hit = &h->graphs.back();
             }
         }
@@ -436,11 +617,12 @@ int neon_svgf_denoise(neon_svgf_handle* h, const float* position, const float* n
         }
     }
     if (!graphs) {
-        const int n = record_frame(h, fr, pp, st);
+        const int n = record_frame(h, fr, pp, ca, st);
         if (n < 0) return sfail(h, NEON_MOE_ECUDA, "kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
         h->launches += n;
     }
     h->ping_pong = !pp;
+    h->cur_a = ca ^ 1;
     h->last_stream = st;
     return NEON_MOE_OK;
 }
@@ -477,7 +659,7 @@ int neon_svgf_read(neon_svgf_handle* h, const char* name, void* dst, uint64_t by
     size_t need = 0;
     if (!strcmp(name, "colour_a")) { src = h->colour_a; need = px * 8; }
     else if (!strcmp(name, "colour_b")) { src = h->colour_b; need = px * 8; }
-    else if (!strcmp(name, "moments")) { src = h->data[0]; need = px * 16; }
+    else if (!strcmp(name, "moments")) need = px * 16;
     else if (!strcmp(name, "ping_pong")) {
         if (bytes != 4) return sfail(h, NEON_MOE_EINVAL, "ping_pong is 4 bytes");
         const int32_t v = h->ping_pong;
@@ -485,6 +667,16 @@ int neon_svgf_read(neon_svgf_handle* h, const char* name, void* dst, uint64_t by
         return NEON_MOE_OK;
     } else return sfail(h, NEON_MOE_EINVAL, "unknown buffer '%s'", name);
     if (bytes != need) return sfail(h, NEON_MOE_EINVAL, "%s is %zu bytes, not %llu", name, need, (unsigned long long)bytes);
+    if (!src) {  // the moments: joined from their planes
+        float4* tmp = nullptr;
+        SCU(h, cudaMalloc(&tmp, px * 16));
+        k_join_moments<<<(unsigned)((px + 255) / 256), 256, 0, h->own_stream>>>(px, h->mom_a[h->cur_a], h->mom_b[0], tmp);
+        cudaError_t e = cudaStreamSynchronize(h->own_stream);
+        if (e == cudaSuccess) e = cudaMemcpy(dst, tmp, need, cudaMemcpyDeviceToHost);
+        cudaFree(tmp);
+        if (e != cudaSuccess) return sfail(h, NEON_MOE_ECUDA, "reading the moments failed: %s", cudaGetErrorString(e));
+        return NEON_MOE_OK;
+    }
     SCU(h, cudaMemcpy(dst, src, need, cudaMemcpyDeviceToHost));
     return NEON_MOE_OK;
 }
@@ -500,12 +692,13 @@ int neon_svgf_profile_frame(neon_svgf_handle* h, const float* position, const fl
                    reinterpret_cast<uchar4*>(image)};
     cudaEvent_t ev[3];
     for (auto& e : ev) SCU(h, cudaEventCreate(&e));
-    const int n = record_frame(h, fr, h->ping_pong, st, ev);
+    const int n = record_frame(h, fr, h->ping_pong, h->cur_a, st, ev);
     int rc = NEON_MOE_OK;
     if (n < 0 || cudaStreamSynchronize(st) != cudaSuccess) rc = sfail(h, NEON_MOE_ECUDA, "profiled frame failed: %s", cudaGetErrorString(cudaGetLastError()));
     else {
         h->launches += n;
         h->ping_pong = !h->ping_pong;
+        h->cur_a ^= 1;
         h->last_stream = st;
         for (int i = 0; i < 2; ++i) {
             float ms = 0.0f;
