@@ -5,6 +5,7 @@
 #include "../../include/neon_pt.h"
 
 #include <cuda_runtime.h>
+#include <xmmintrin.h>
 
 #include <algorithm>
 #include <cmath>
@@ -374,77 +375,89 @@ __global__ void __launch_bounds__(64) pt_frame_kernel(Scene sc, Camera cam, int 
 }
 
 // ---- host: hierarchy construction -----------------------------------------------------------------------
-// Splits by the surface area heuristic over 16 bins per axis, leaves of at most kLeaf triangles (fewer where splitting
+// Splits by the surface area heuristic over up to 16 bins per axis (fewer for few triangles, where sweeping the bins is
+// the cost), leaves of at most kLeaf triangles (fewer where splitting
 // costs less); from kSahDepth levels on, and where all centroids fall into one bin, by the median of the longest
 // centroid axis, so that the depth stays below the traversal's stack.
-constexpr int kLeaf = 4, kBins = 16, kSahDepth = 20, kMaxDepthBvh = kStack - 4;
+constexpr int kLeaf = 4, kBins = 16, kSample = 512, kSahDepth = 20, kMaxDepthBvh = kStack - 4;
 constexpr float kNodeCost = 1.5f;  // one node visit in units of one triangle test
 
-struct Box {
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    void add(const float* l, const float* h) {
-        for (int a = 0; a < 3; ++a) { lo[a] = std::min(lo[a], l[a]); hi[a] = std::max(hi[a], h[a]); }
-    }
+struct Box {  // four lanes, three of them used; a NaN coordinate leaves a bound as it is
+    __m128 lo = _mm_set1_ps(INFINITY), hi = _mm_set1_ps(-INFINITY);
+    void add(const Box& b) { lo = _mm_min_ps(b.lo, lo); hi = _mm_max_ps(b.hi, hi); }
     float area() const {
-        const float x = hi[0] - lo[0], y = hi[1] - lo[1], z = hi[2] - lo[2];
-        return x >= 0.f ? x * y + y * z + z * x : 0.f;  // nothing added yet: empty
+        alignas(16) float e[4];
+        _mm_store_ps(e, _mm_sub_ps(hi, lo));
+        return e[0] >= 0.f ? e[0] * e[1] + e[1] * e[2] + e[2] * e[0] : 0.f;  // nothing added yet: empty
     }
 };
 
 struct Builder {
     std::vector<BvhNode> nodes;
     std::vector<int> order;
-    std::vector<float> cmin, cmax, cen;  // per triangle: bounds and centroid (3 floats each)
-    std::vector<uint8_t> last;           // per place in `order`: the last triangle of its leaf
-    int max_depth = 0, n_nodes = 0;      // nodes in the usual sense: inner nodes and leaves
+    std::vector<Box> tri;       // per triangle: its bounds
+    std::vector<Box> cen;       // and its centroid (both bounds)
+    std::vector<uint8_t> last;  // per place in `order`: the last triangle of its leaf
+    int max_depth = 0, n_nodes = 0;  // nodes in the usual sense: inner nodes and leaves
+    Box bin_boxes[3][kBins];
 
+    float centroid(int t, int a) const { return reinterpret_cast<const float*>(&cen[t].lo)[a]; }
     Box bounds(int first, int count) const {
         Box b;
-        for (int i = first; i < first + count; ++i) b.add(&cmin[3 * (size_t)order[i]], &cmax[3 * (size_t)order[i]]);
+        for (int i = first; i < first + count; ++i) b.add(tri[order[i]]);
         return b;
     }
     // the place to cut [first, first + count) at after reordering it, or first for a leaf
     int split(int first, int count, int depth, const Box& box) {
         if (count <= 1 || depth >= kMaxDepthBvh) return first;
-        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-        for (int i = first; i < first + count; ++i)
-            for (int a = 0; a < 3; ++a) {
-                const float c = cen[3 * (size_t)order[i] + a];
-                lo[a] = std::min(lo[a], c);
-                hi[a] = std::max(hi[a], c);
-            }
+        Box c;
+        for (int i = first; i < first + count; ++i) c.add(cen[order[i]]);
+        alignas(16) float lo[4], hi[4];
+        _mm_store_ps(lo, c.lo);
+        _mm_store_ps(hi, c.hi);
+        const int n_bins = std::min(kBins, std::max(4, count));
+        float scale[3];
+        for (int a = 0; a < 3; ++a) scale[a] = (float)n_bins / (hi[a] - lo[a]);
+        auto bin_of = [&](int t, int a) {
+            const float f = (centroid(t, a) - lo[a]) * scale[a];
+            return f > 0.f ? std::min(n_bins - 1, (int)std::min(f, (float)n_bins)) : 0;  // also where a coordinate is not finite
+        };
         int best_axis = -1, best_bin = 0;
         float best_cost = INFINITY;
-        auto bin_of = [&](int t, int a) {
-            const float f = (cen[3 * (size_t)t + a] - lo[a]) / (hi[a] - lo[a]) * (float)kBins;
-            return f > 0.f ? std::min(kBins - 1, (int)std::min(f, (float)kBins)) : 0;  // also where a coordinate is not finite
-        };
-        if (depth < kSahDepth)
+        if (depth < kSahDepth) {
+            Box (*bins)[kBins] = bin_boxes;  // scratch: only the bins in use are cleared
+            int n[3][kBins];
+            // many triangles: about kSample of them, evenly spread
+            const int step = std::max(1, count / kSample), sampled = (count + step - 1) / step;
+            for (int a = 0; a < 3; ++a)
+                for (int b = 0; b < n_bins; ++b) { bins[a][b] = Box(); n[a][b] = 0; }
+            for (int i = first; i < first + count; i += step) {
+                const int t = order[i];
+                for (int a = 0; a < 3; ++a) {
+                    const int b = bin_of(t, a);
+                    bins[a][b].add(tri[t]);
+                    ++n[a][b];
+                }
+            }
             for (int a = 0; a < 3; ++a) {
                 if (!(hi[a] > lo[a])) continue;
-                Box bins[kBins];
-                int n[kBins] = {};
-                for (int i = first; i < first + count; ++i) {
-                    const int b = bin_of(order[i], a);
-                    bins[b].add(&cmin[3 * (size_t)order[i]], &cmax[3 * (size_t)order[i]]);
-                    ++n[b];
-                }
                 float right_area[kBins];
                 Box acc;
-                for (int b = kBins - 1; b > 0; --b) {
-                    acc.add(bins[b].lo, bins[b].hi);
+                for (int b = n_bins - 1; b > 0; --b) {
+                    acc.add(bins[a][b]);
                     right_area[b] = acc.area();
                 }
                 acc = Box();
                 int left = 0;
-                for (int b = 0; b + 1 < kBins; ++b) {
-                    acc.add(bins[b].lo, bins[b].hi);
-                    left += n[b];
-                    if (!left || left == count) continue;
-                    const float cost = acc.area() * (float)left + right_area[b + 1] * (float)(count - left);
+                for (int b = 0; b + 1 < n_bins; ++b) {
+                    acc.add(bins[a][b]);
+                    left += n[a][b];
+                    if (!left || left == sampled) continue;
+                    const float cost = acc.area() * (float)left + right_area[b + 1] * (float)(sampled - left);
                     if (cost < best_cost) { best_cost = cost; best_axis = a; best_bin = b; }
                 }
             }
+        }
         if (best_axis >= 0) {
             if (count <= kLeaf && best_cost + kNodeCost * box.area() >= box.area() * (float)count) return first;
             const auto mid = std::partition(order.begin() + first, order.begin() + first + count, [&](int t) { return bin_of(t, best_axis) <= best_bin; });
@@ -456,7 +469,7 @@ struct Builder {
         if (hi[2] - lo[2] > hi[axis] - lo[axis]) axis = 2;
         const int mid = first + count / 2;
         std::nth_element(order.begin() + first, order.begin() + mid, order.begin() + first + count, [&](int a, int b) {
-            const float ca = cen[3 * (size_t)a + axis], cb = cen[3 * (size_t)b + axis];
+            const float ca = centroid(a, axis), cb = centroid(b, axis);
             return ca < cb || (ca == cb && a < b);
         });
         return mid;
@@ -476,11 +489,14 @@ struct Builder {
             const Box b = bounds(f, n);
             const int ref = build(f, n, depth + 1, b);
             nodes[node].ref[c] = ref;
+            alignas(16) float lo[4], hi[4];
+            _mm_store_ps(lo, b.lo);
+            _mm_store_ps(hi, b.hi);
             for (int a = 0; a < 3; ++a) {  // padded: the slab test must never lose a hit that lies on a face
-                const float pad = 1e-5f * std::max(1.f, std::max(std::fabs(b.lo[a]), std::fabs(b.hi[a])));
+                const float pad = 1e-5f * std::max(1.f, std::max(std::fabs(lo[a]), std::fabs(hi[a])));
                 float* side = a == 0 ? nodes[node].x : (a == 1 ? nodes[node].y : nodes[node].z);
-                side[2 * c] = b.lo[a] - pad;
-                side[2 * c + 1] = b.hi[a] + pad;
+                side[2 * c] = lo[a] - pad;
+                side[2 * c + 1] = hi[a] + pad;
             }
         }
         return node;
@@ -557,15 +573,18 @@ int neon_pt_create(const neon_pt_config* cfg, const neon_pt_vertex* vertices, in
     const int n_tri = n_indices / 3;
     Builder b;
     b.order.resize(n_tri);
-    b.cmin.resize(3 * (size_t)n_tri); b.cmax.resize(3 * (size_t)n_tri); b.cen.resize(3 * (size_t)n_tri);
+    b.tri.resize(n_tri);
+    b.cen.resize(n_tri);
     for (int t = 0; t < n_tri; ++t) {
         b.order[t] = t;
-        for (int a = 0; a < 3; ++a) {
-            const float p0 = vertices[indices[3 * t]].pos[a], p1 = vertices[indices[3 * t + 1]].pos[a], p2 = vertices[indices[3 * t + 2]].pos[a];
-            b.cmin[3 * t + a] = std::min(p0, std::min(p1, p2));
-            b.cmax[3 * t + a] = std::max(p0, std::max(p1, p2));
-            b.cen[3 * t + a] = (p0 + p1 + p2) * (1.f / 3.f);
+        __m128 p[3];
+        for (int c = 0; c < 3; ++c) {
+            const float* v = vertices[indices[3 * t + c]].pos;
+            p[c] = _mm_set_ps(0.f, v[2], v[1], v[0]);
+            b.tri[t].lo = c ? _mm_min_ps(p[c], b.tri[t].lo) : p[c];
+            b.tri[t].hi = c ? _mm_max_ps(p[c], b.tri[t].hi) : p[c];
         }
+        b.cen[t].lo = b.cen[t].hi = _mm_mul_ps(_mm_add_ps(_mm_add_ps(p[0], p[1]), p[2]), _mm_set1_ps(1.f / 3.f));
     }
     b.last.resize(n_tri);
     b.nodes.reserve(n_tri);
