@@ -1037,13 +1037,13 @@ def moe_roofline(run, step_s, stage_ms, n_prof, peaks, peak_kind, traffic_table)
     layer_bytes = mean_touched * shape.expert_bytes + shape.router_bytes + T * H * 2 + T * H * 4
     gu_expert_bytes = 2 * I * H // 2 + 2 * I * H // 32 + 2 * I * 2
     if run.layer.launch_count and T <= 8 and stage_ms is None:
-        # one cooperative kernel per pass: the kernel is the layer, its algorithmic bytes are the layer's
+        # the pass is measured as a whole: its algorithmic bytes are the layer's
         achieved = layer_bytes / step_s / 1e9
-        roof = {"bound": "hbm", "kernel": "decode_fused_kernel (router + gate_up + SwiGLU + down + combine, one launch)",
+        roof = {"bound": "hbm", "kernel": "stream_route_kernel + stream_gate_up_kernel + stream_down_kernel" if T == 1 else "the whole pass",
                 "achieved": achieved, "peak": peaks["hbm_gbs"], "peak_kind": peak_kind, "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": None, "algorithmic_bytes_per_launch": layer_bytes,
                 "ms_per_launch": step_s * 1e3,
-                "note": "launch duration = the step (one kernel per pass, replayed from a CUDA graph; CUDA events around K passes)"}
+                "note": "launch duration = the step (the pass's kernels, replayed from a CUDA graph; CUDA events around K passes)"}
     elif run.decode:
         gu_ms = stage_ms["gate_up"]
         gu_bytes = mean_touched * gu_expert_bytes + T * H * 2 + T * k * I * 4

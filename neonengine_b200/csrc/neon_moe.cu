@@ -19,6 +19,7 @@
 #include "ep.cuh"
 #include "decode_fused.cuh"
 #include "decode_sliced.cuh"
+#include "decode_stream.cuh"
 #include "gmm_pair_prefill_sm100.cuh"
 #include "mma_rate.cuh"
 #include "mma_pair.cuh"
@@ -82,7 +83,7 @@ struct neon_moe_handle {
     int decode_sliced = 0;        // 1 = the one-launch pass runs sliced by intermediate channel (decode_sliced.cuh) where it can; measured no faster
     int decode_fused = 1;         // 1 = passes of at most decode_fused_tokens tokens run as one cooperative kernel
     int decode_max_tokens = 0;    // largest pass the one-launch kernel can serve on this handle (0 = not available)
-    int decode_fused_tokens = 1;  // largest pass it serves by default: measured per pass at the gpt-oss-20b shapes, one launch vs
+    int decode_fused_tokens = 1;  // largest pass it serves (at 1, one token goes to decode_stream's kernels where they are on): measured per pass at the gpt-oss-20b shapes, one launch vs
                                   // the multi-kernel path: T=1 36.5 vs 38.7 us, T=2 51 vs 49, T=8 129 vs 79 (more distinct experts per
                                   // CTA run: more rebuilds of the token-operand tiles, longer combine)
     int decode_stall_test = 0;    // test hook: the kernel's first wait expects one arrival too many and must time out
@@ -95,6 +96,10 @@ struct neon_moe_handle {
     int dec_sliced_tokens = 0;    // largest pass decode_sliced_kernel can take (0: unavailable)
     unsigned* dec_counters = nullptr;
     int dec_gu_items_cap = 0, dec_counter_words = 0;
+    int decode_stream = 1;        // 1 = a pass of one token runs as a plain weight stream (decode_stream.cuh)
+    bool stream_ready = false;    // this handle has what that takes
+    __half *str_x = nullptr, *str_a = nullptr;
+    StreamTables* str_tab = nullptr;
     int pair_ctas = 0;            // CTAs the paired kernel was last launched with (2 x resident clusters)
     // Decode tiles (16 / 32 tokens) on clusters of two CTAs with two-SM MMAs (tcgen05 cta_group::2): 0 never, 1 always,
     // 2 when the pass routes at most kPairMaxEntries entries.  Measured per pass at the gpt-oss shapes, single vs paired
@@ -206,7 +211,7 @@ int dev_alloc(neon_moe_handle* h, T** p, size_t count) {
 }
 
 void free_all(neon_moe_handle* h) {
-    void* ptrs[] = {h->router_w, h->router_b, h->gu_bias, h->dn_bias, h->gu_wq, h->dn_wq, h->gu_sq, h->dn_sq,
+    void* ptrs[] = {h->str_x, h->str_a, h->str_tab, h->router_w, h->router_b, h->gu_bias, h->dn_bias, h->gu_wq, h->dn_wq, h->gu_sq, h->dn_sq,
                     h->idx, h->count, h->offset, h->perm, h->inv, h->route_w, h->y, h->a_hi, h->a_lo,
                     h->status, h->st_hidden, h->st_out, h->st_bias, h->st_hidden2, h->st_out2, h->gu_wt, h->gu_sfa, h->dn_wt, h->dn_sfa,
                     h->x_act, h->a_act, h->x_scale, h->x_amax, h->a_f32, h->tile_expert, h->tile_row0, h->tile_rows,
@@ -817,6 +822,16 @@ int neon_moe_create(const neon_moe_config* cfg, neon_moe_handle** out) {
             h->dec_sliced_tokens = t2;
         }
     }
+    // the streamed pass of one token: one GPU holding all experts
+    if (h->path == 2 && cfg->ep_size == 1) {
+        const size_t nx = (size_t)h->kp_h, na = (size_t)cfg->top_k * 2 * h->kp_i;
+        if ((rc = dev_alloc(h, &h->str_x, nx)) || (rc = dev_alloc(h, &h->str_a, na)) || (rc = dev_alloc(h, &h->str_tab, (size_t)1))) return bail(rc);
+        // the columns between the depth and its padding are never written: they stay zero
+        if (cudaMemset(h->str_x, 0, nx * 2) != cudaSuccess || cudaMemset(h->str_a, 0, na * 2) != cudaSuccess ||
+            cudaMemset(h->str_tab, 0, sizeof(StreamTables)) != cudaSuccess)
+            return bail(fail(h, NEON_MOE_ECUDA, "cudaMemset failed"));
+        h->stream_ready = true;
+    }
     if (cfg->ep_size > 1) {
         const size_t ns = (size_t)h->n_src, E = (size_t)cfg->n_experts, Hh = (size_t)cfg->hidden;
         if ((rc = dev_alloc(h, &h->s_idx, ns)) || (rc = dev_alloc(h, &h->s_w, ns)) || (rc = dev_alloc(h, &h->s_count, E)) ||
@@ -1084,6 +1099,52 @@ static int launch_decode_sliced(neon_moe_handle* h, const void* hidden, int T, c
     return NEON_MOE_OK;
 }
 
+// A pass of one token as three kernels that stream weights (decode_stream.cuh).
+static int launch_decode_stream(neon_moe_handle* h, const void* hidden, const float* logit_bias, float* out, cudaStream_t st) {
+    const int H = h->cfg.hidden, I = h->cfg.inter, E = h->cfg.n_experts;
+    StreamParams p{};
+    p.x = static_cast<const uint16_t*>(hidden); p.wr = h->router_w; p.br = h->router_b; p.logit_bias = logit_bias;
+    p.H = H; p.I = I; p.E = E; p.k = h->cfg.top_k; p.kp_h = h->kp_h; p.kp_i = h->kp_i; p.dn_tiles = (H + 127) / 128;
+    p.limit = h->cfg.swiglu_limit; p.alpha = h->cfg.swiglu_alpha;
+    p.gu_w = h->gu_wt; p.gu_sfa = h->gu_sfa; p.dn_w = h->dn_wt; p.dn_sfa = h->dn_sfa; p.gu_bias = h->gu_bias; p.dn_bias = h->dn_bias;
+    p.n_slices = std::max(1, std::min(kStrSlicesMax, kStrCluster * (kStrRouteThreads / 32) / E));
+    {   // |SwiGLU| <= limit * (limit + 1), which goes to [2^14, 2^15); kept where the factor and its inverse are normal
+        const float bound = h->cfg.swiglu_limit * (h->cfg.swiglu_limit + 1.f);
+        uint32_t bits;
+        memcpy(&bits, &bound, 4);
+        bits = (uint32_t)std::min(std::max(268 - (int)((bits >> 23) & 0xffu), 1), 253) << 23;
+        memcpy(&p.a_inv, &bits, 4);
+    }
+    p.xt = h->str_x; p.at = h->str_a; p.tab = h->str_tab;
+    p.out = out; p.idx = h->idx; p.route_w = h->route_w;
+    p.d = DispatchArrays{h->count, h->offset, h->perm, h->inv};
+    static bool configured[kMaxDevicesAttr] = {};
+    if (!configured[h->cfg.device]) {
+        CU(h, cudaFuncSetAttribute(stream_gate_up_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrGuSmem));
+        CU(h, cudaFuncSetAttribute(stream_down_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrDnSmem));
+        configured[h->cfg.device] = true;
+    }
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    cfg.gridDim = dim3(kStrCluster);
+    cfg.blockDim = dim3(kStrRouteThreads);
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kStrCluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = h->pdl ? 2 : 1;
+    CU(h, cudaLaunchKernelEx(&cfg, stream_route_kernel, p));
+    const int items = p.k * (2 * I / 128) * 4;
+    launch_k(h->pdl != 0, stream_gate_up_kernel, dim3(std::min(items, h->n_sms * 5)), dim3(kStrGuWarps * 32), (size_t)kStrGuSmem, st, p);
+    launch_k(h->pdl != 0, stream_down_kernel, dim3(p.dn_tiles * 8), dim3(kStrDnWarps * 32), (size_t)kStrDnSmem, st, p);
+    h->launches += 3;
+    CU(h, cudaGetLastError());
+    return NEON_MOE_OK;
+}
+
 static void launch_router(neon_moe_handle* h, const void* hidden, int T, const float* logit_bias, int32_t* idx, float* w,
                           float* tok_amax, cudaStream_t st) {
     const int H = h->cfg.hidden, E = h->cfg.n_experts, k = h->cfg.top_k;
@@ -1189,9 +1250,13 @@ static int forward_eager(neon_moe_handle* h, const void* hidden, int T, const fl
     CU(h, cudaSetDevice(h->cfg.device));
     const int k = h->cfg.top_k, n = T * k;
     const bool prof = h->profiling && h->events_used + 5 <= 5 * kMaxProfiledForwards;
-    if (h->path == 2 && h->decode_fused && T <= std::min(h->decode_max_tokens, h->decode_fused_tokens) && !prof && h->tile_override == 0 && !h->mx4 && !h->fuse_dispatch) {
-        int rc = (h->decode_sliced && T <= h->dec_sliced_tokens) ? launch_decode_sliced(h, hidden, T, logit_bias, out, st)
-                                                                  : launch_decode_fused(h, hidden, T, logit_bias, out, st);
+    const bool small = h->path == 2 && h->decode_fused && !prof && h->tile_override == 0 && !h->mx4 && !h->fuse_dispatch;
+    const bool streamed = small && T == 1 && h->decode_stream && h->stream_ready && h->decode_fused_tokens <= 1;
+    const bool one_launch = small && !streamed && T <= std::min(h->decode_max_tokens, h->decode_fused_tokens);
+    if (streamed || one_launch) {
+        int rc = streamed ? launch_decode_stream(h, hidden, logit_bias, out, st)
+                 : (h->decode_sliced && T <= h->dec_sliced_tokens) ? launch_decode_sliced(h, hidden, T, logit_bias, out, st)
+                                                                   : launch_decode_fused(h, hidden, T, logit_bias, out, st);
         if (rc) return rc;
         if (topk_idx) CU(h, cudaMemcpyAsync(topk_idx, h->idx, (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
         if (topk_w) CU(h, cudaMemcpyAsync(topk_w, h->route_w, (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
@@ -1648,6 +1713,9 @@ int neon_moe_set_option(neon_moe_handle* h, const char* name, int64_t value) {
     } else if (!strcmp(name, "decode_fused_tokens")) {
         if (value < 0 || value > kDecMaxTok) return fail(h, NEON_MOE_EINVAL, "decode_fused_tokens must lie in [0, %d]", kDecMaxTok);
         h->decode_fused_tokens = (int)value;
+    } else if (!strcmp(name, "decode_stream")) {
+        h->decode_stream = value != 0;
+        drop_graphs(h);
     } else if (!strcmp(name, "decode_stall_test")) {
         h->decode_stall_test = (int)value;
     } else if (!strcmp(name, "decode_wait_limit")) {

@@ -1,0 +1,49 @@
+"""GPU parity of the streamed pass of one token (csrc/decode_stream.cuh): depths whose chunks do not divide evenly
+over its warps (fewer chunks than warps among them), a last weight tile that is half padding, every expert count that
+changes the router's split, scale bytes over a wide range, a token whose logits are the bias alone, against the CPU
+oracle and against the one-launch and the grouped-GEMM path."""
+import numpy as np
+import pytest
+
+import oracle
+from helpers import assert_close, errors
+from neonengine_b200 import synth
+from test_moe_gpu import check_against_oracle, make_layer, run_device
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("hidden,inter,experts,top_k", [(64, 64, 8, 2), (192, 320, 32, 4), (576, 192, 128, 4), (704, 448, 256, 3), (320, 576, 4, 4), (2880, 64, 8, 8)])
+@pytest.mark.parametrize("seed", [1, 2])
+def test_against_the_oracle(hidden, inter, experts, top_k, seed):
+    shape = synth.MoeShape(hidden=hidden, inter=inter, n_experts=experts, top_k=top_k)
+    W = synth.make_weights(shape, 11)
+    lb = synth.zipf_logit_bias(experts) if seed == 2 and experts > top_k else None
+    x = synth.make_hidden(1, W, 20 + seed, logit_bias=lb)
+    layer = make_layer(shape, W, max_tokens=8)
+    layer.set_option("use_graphs", 0)
+    before = layer.launch_count
+    out, (max_abs, mean_rel) = check_against_oracle(layer, W, x, logit_bias=lb, what="stream")
+    assert layer.launch_count - before == 3
+    # f32 sums of at most 2880 exact products (their rounding adds up like its square root, 54 * 2^-24) and 22-bit activations
+    assert mean_rel < 4e-6, (max_abs, mean_rel)
+    np.testing.assert_array_equal(run_device(layer, x, lb)[0], out)  # two runs, the same bits
+    for option, launches in (("decode_stream", 1), ("decode_fused", 6)):
+        layer.set_option(option, 0)
+        before = layer.launch_count
+        assert_close(out, run_device(layer, x, lb)[0], "stream vs " + option + " 0")
+        assert layer.launch_count - before >= launches
+    layer.close()
+
+
+def test_scales_over_a_wide_range_and_a_zero_token():
+    shape = synth.MoeShape(hidden=192, inter=128, n_experts=8, top_k=2)
+    W = synth.make_weights(shape, 3)
+    rng = np.random.default_rng(0)
+    W.gate_up_scales[:] = rng.integers(2, 132, W.gate_up_scales.shape)
+    W.down_scales[:] = rng.integers(2, 132, W.down_scales.shape)
+    layer = make_layer(shape, W, max_tokens=1)
+    for x in (synth.make_hidden(1, W, 5), np.zeros((1, 192), np.uint16)):
+        out, idx, w = run_device(layer, x)
+        assert errors(out, oracle.experts(x, idx, w, W))[1] < 4e-6 and np.isfinite(out).all()
+    layer.close()
