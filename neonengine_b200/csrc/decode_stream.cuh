@@ -121,39 +121,6 @@ constexpr int kStrGuStages = 4, kStrDnStages = 4;
 constexpr int kStrGuSmem = kStrGuWarps * kStrGuStages * StreamRing<2, 1>::kStage, kStrDnSmem = kStrDnWarps * kStrDnStages * StreamRing<1, 2>::kStage;
 
 // ---- routing ------------------------------------------------------------------------------------------------------
-// Top k of the logits (lgt[E] in shared memory), ties to the lower expert id, softmax over the selected ones; one warp.
-// Same selection as dec_topk_warp, on 32-bit keys with the warp's own reductions.
-__device__ __forceinline__ void stream_topk_warp(const float* lgt, int E, int k, int lane, int* idx_out, float* w_out) {
-    constexpr int J = kMaxExperts / 32;
-    uint32_t key[J];
-#pragma unroll
-    for (int j = 0; j < J; ++j) {
-        const int e = lane + 32 * j;
-        key[j] = e < E ? (uint32_t)(logit_key(lgt[e], e) >> 32) : 0u;  // 0 is below every number's key
-    }
-    float first = 0.f, den = 0.f, mine = 0.f;
-    for (int s = 0; s < k; ++s) {
-        uint32_t best = 0u;
-#pragma unroll
-        for (int j = 0; j < J; ++j) best = max(best, key[j]);
-        best = __reduce_max_sync(0xffffffffu, best);
-        int e = 0x7fffffff;
-#pragma unroll
-        for (int j = J - 1; j >= 0; --j)
-            if (key[j] == best && lane + 32 * j < E) e = lane + 32 * j;
-        e = __reduce_min_sync(0xffffffffu, e);
-#pragma unroll
-        for (int j = 0; j < J; ++j)
-            if (lane + 32 * j == e) key[j] = 0u;
-        const float l = lgt[e];
-        if (s == 0) first = l;
-        const float pr = expf(l - first);
-        den += pr;
-        if (lane == s) { mine = pr; idx_out[s] = e; }
-    }
-    if (lane < k) w_out[lane] = mine / den;
-}
-
 __global__ void __launch_bounds__(kStrRouteThreads) stream_route_kernel(const StreamParams p) {
     __shared__ float part[kMaxExperts * kStrSlicesMax], lg[kMaxExperts];  // CTA 0: the shares of the logits, the logits
     __shared__ unsigned amax;
@@ -239,7 +206,7 @@ __global__ void __launch_bounds__(kStrRouteThreads) stream_route_kernel(const St
         lg[e] = v;
     }
     __syncthreads();
-    if (warp == 0) stream_topk_warp(lg, E, k, lane, s_idx, s_w);
+    if (warp == 0) topk_warp(lg, E, k, lane, s_idx, s_w);
     __syncthreads();
     if (tid < k) {
         const int e = s_idx[tid];

@@ -62,9 +62,8 @@ struct neon_moe_handle {
     int max_stages = 0, ctas_per_sm = 1;
     int pdl = 1;                  // programmatic dependent launch between the kernels of a pass
     int tile_override = 0;        // 0 = token-tile size chosen from the batch size; 16 / 32 / 128 force it
-    int router_wide_max = 384;    // passes up to this many tokens use the one-CTA-per-token router, which also yields the token
-                                  // maxima the stacked-term tiles need (measured 9-13 us faster than the token-blocked router
-                                  // plus a separate maxima kernel at 96-256 tokens, equal at 384)
+    int router_wide_max = 224;    // passes up to this many tokens use the one-CTA-per-token router, which also yields the token
+                                  // maxima the stacked-term tiles need - which passes of up to 224 tokens run on
     int graph_max_tokens = 64;    // passes up to this many tokens are replayed from a captured CUDA graph
     int router_mma = 1;           // larger passes route on tensor cores (32 or 128 experts); 0 = the token-blocked CUDA-core router
     int sync_debug = 0;           // synchronise and check after every kernel (slow; names the failing kernel)
@@ -517,6 +516,20 @@ int launch_gmm_pair_prefill(neon_moe_handle* h, const CUtensorMap& tm1, GmmParam
 constexpr int kDownTermsPrefill = 3;
 constexpr int kDecodeSmemBytes = 227 * 1024;  // everything an SM has: what the token-operand tiles leave goes to weight stages
 constexpr int kPairMaxEntries = 128 * 4;  // passes of up to 128 tokens at top-4 take the paired kernel
+template <int MT, int U>
+void launch_router_mma(neon_moe_handle* h, const void* hidden, int T, const float* logit_bias, int32_t* idx, float* w, cudaStream_t st) {
+    const int E = h->cfg.n_experts, tokens = 16 * MT;
+    static bool configured[kMaxDevicesAttr] = {};
+    if (!configured[h->cfg.device]) {
+        cudaFuncSetAttribute(router_topk_mma_kernel<MT, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, MT * 32 * 1024);
+        configured[h->cfg.device] = true;
+    }
+    const size_t smem = (size_t)(kRouterMmaWarps / (E / 32)) * tokens * E * sizeof(float);  // 32 KB per 16 tokens
+    launch_k(h->pdl != 0, router_topk_mma_kernel<MT, U>, dim3((T + tokens - 1) / tokens), dim3(kRouterMmaWarps * 32), smem, st,
+             static_cast<const uint16_t*>(hidden), (const uint16_t*)h->router_w, (const uint16_t*)h->router_b, logit_bias, T, h->cfg.hidden, E,
+             h->cfg.top_k, idx, w);
+}
+
 constexpr int kMx4Terms = 6;  // e2m1 terms per activation value on the packed 4-bit path
 
 template <int TERMS, bool GATE_UP>
@@ -1149,16 +1162,10 @@ static void launch_router(neon_moe_handle* h, const void* hidden, int T, const f
                           float* tok_amax, cudaStream_t st) {
     const int H = h->cfg.hidden, E = h->cfg.n_experts, k = h->cfg.top_k;
     if (h->path == 2 && T > h->router_wide_max && h->router_mma && (E == 32 || E == 128) && H % 32 == 0) {
-        // tensor-core router, 16 tokens per CTA: no token maxima (128-token tiles scale per block)
-        const size_t smem = (size_t)4 * 16 * E * sizeof(float);
-        if (E == 32)
-            launch_k(h->pdl != 0, router_topk_mma_kernel<4>, dim3((T + 15) / 16), dim3(128), smem, st,
-                     static_cast<const uint16_t*>(hidden), (const uint16_t*)h->router_w, (const uint16_t*)h->router_b, logit_bias, T,
-                     H, k, idx, w);
-        else
-            launch_k(h->pdl != 0, router_topk_mma_kernel<16>, dim3((T + 15) / 16), dim3(128), smem, st,
-                     static_cast<const uint16_t*>(hidden), (const uint16_t*)h->router_w, (const uint16_t*)h->router_b, logit_bias, T,
-                     H, k, idx, w);
+        // tensor-core router: no token maxima (128-token tiles scale per block); token tiles that leave the CTAs one wave
+        if (T <= 16 * h->n_sms) launch_router_mma<1, 3>(h, hidden, T, logit_bias, idx, w, st);
+        else if (T <= 32 * h->n_sms) launch_router_mma<2, 2>(h, hidden, T, logit_bias, idx, w, st);
+        else launch_router_mma<4, 1>(h, hidden, T, logit_bias, idx, w, st);
     } else if (h->path == 2 && T > h->router_wide_max) {  // token-blocked router: no token maxima either
         const size_t smem = (size_t)8 * H * 2 + (size_t)8 * E * sizeof(float);
         static bool configured[kMaxDevicesAttr] = {};
