@@ -507,130 +507,82 @@ __host__ __device__ inline size_t act_block_bytes(int terms, int tile_tokens, bo
     return (size_t)act_header_bytes(terms) + (size_t)(tile_tokens / 8) * terms * 1024;
 }
 
-// ---- prefill operand rows -------------------------------------------------------------------------------------------
-// One warp per (source row, group of kSplitChunksPerWarp chunks): 16 lanes per chunk, 8 elements a lane, all loads issued
-// before any arithmetic.  A token's hidden state is written once for each of its top_k entries but worked out once
-// (FROM_BF16: source row = token, its entries' sorted positions from inv; otherwise source row = sorted row).  Bound by the
-// instructions per element (scales, conversions, remainders), then by the bytes written.  One warp a chunk with 4 elements
-// a lane and the terms worked out again for every entry took 58 us (two terms of 16384 entries) and 80 us (three terms of
-// the SwiGLU rows) of a 4096-token pass; with this split the whole pass went from 1120 to 1073 us, with 4-bit activations
-// (whose kernel had loaded one chunk a warp) from 632 to 570 us, and 300 tokens are unchanged.
+// Chunks one warp of split_rows_kernel handles (all their loads are issued before any arithmetic).
 constexpr int kSplitChunksPerWarp = 4;
 
-struct SplitPlace {  // lane s: token tile and row in it of the source row's copy s (row < 0: none)
-    int tile, row;
-};
-template <bool FROM_BF16>
-__device__ __forceinline__ SplitPlace split_places(int r, int top_k, int n_rows, const int32_t* inv, const int32_t* row_tile,
-                                                   const int32_t* tile_row0, int lane) {
-    SplitPlace at{0, -1};
-    if (lane < (FROM_BF16 ? top_k : 1)) {
-        const int p = FROM_BF16 ? inv[r * top_k + lane] : r;
-        if (p >= 0 && p < n_rows) {
-            at.tile = row_tile[p];
-            at.row = p - tile_row0[at.tile];
-        }
-    }
-    return at;
-}
-// The 8 elements of a row from column k0 on (zeros beyond K).
-template <bool FROM_BF16>
-__device__ __forceinline__ void split_load8(const void* src, size_t row, int K, int k0, float (&v)[8]) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = 0.f;
-    if (k0 < K) {  // K % 64 == 0: all eight or none
-        if (FROM_BF16) {
-            const uint4 raw = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(src) + row * K + k0);
-            const uint32_t a[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                v[2 * i] = __uint_as_float(a[i] << 16);
-                v[2 * i + 1] = __uint_as_float(a[i] & 0xffff0000u);
-            }
-        } else {
-            const float4* f = reinterpret_cast<const float4*>(static_cast<const float*>(src) + row * K + k0);
-            const float4 x = f[0], y = f[1];
-            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-            v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
-        }
-    }
-}
-// Largest magnitude of a block of 32: four lanes of eight elements.
-__device__ __forceinline__ float block_amax(const float (&v)[8]) {
-    float m = fabsf(v[0]);
-#pragma unroll
-    for (int i = 1; i < 8; ++i) m = fmaxf(m, fabsf(v[i]));
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    return fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-}
-// The four blocks' scale bytes of this lane's chunk as one word (valid in the chunk's first lane).
-__device__ __forceinline__ uint32_t chunk_scales(uint32_t sb, int lane) {
-    const int base = lane & 16;
-    uint32_t w = sb;
-    w |= __shfl_sync(0xffffffffu, sb, base + 4) << 8;
-    w |= __shfl_sync(0xffffffffu, sb, base + 8) << 16;
-    w |= __shfl_sync(0xffffffffu, sb, base + 12) << 24;
-    return w;
-}
-
-// 128-token tiles: e4m3 terms with a power-of-two scale per block of 32 and term; term t + 1 takes the remainder of term t.
-// Block per (tile, chunk): scale atoms (byte (n % 32) * 16 + (n / 32) * 4 + kb of tile row n, k-block kb) of all terms, then
-// row groups of 8 rows: 128-byte-swizzled K-major rows, terms interleaved group by group.
-template <int TERMS, bool FROM_BF16>
-__global__ void __launch_bounds__(256) split_rows_kernel(const void* __restrict__ src, const int32_t* __restrict__ inv, int top_k, int K,
-                                                         int n_src, int n_rows, const int32_t* __restrict__ row_tile,
-                                                         const int32_t* __restrict__ tile_row0, int tile_tokens, uint8_t* __restrict__ act) {
+template <int TERMS, bool FROM_BF16, bool STACK>
+__global__ void __launch_bounds__(256) split_rows_kernel(const void* __restrict__ src, const int32_t* __restrict__ perm,
+                                                         int top_k, int K, int n_rows, const int32_t* __restrict__ row_tile,
+                                                         const int32_t* __restrict__ tile_row0,
+                                                         const int32_t* __restrict__ tile_rows, int tile_tokens,
+                                                         uint8_t* __restrict__ act) {
     pdl_launch_dependents();
     pdl_wait();
-    constexpr int U = kSplitChunksPerWarp / 2;
-    const int n_chunks = round_up_int(K, kChunkK) / kChunkK, groups = (n_chunks + 2 * U - 1) / (2 * U);
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, l16 = lane & 15;
-    if (warp >= n_src * groups) return;
-    const int r = warp / groups, c0 = (warp % groups) * 2 * U + (lane >> 4);  // this lane's first chunk
-    float vv[U][8];
+    constexpr int U = kSplitChunksPerWarp;
+    const int Kp = round_up_int(K, kChunkK), n_chunks = Kp / kChunkK, groups = (n_chunks + U - 1) / U;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (warp >= n_rows * groups) return;
+    const int p = warp / groups, c0 = (warp % groups) * U;
+    float vv[U][4];
+    {
+        const uint16_t* row16 = nullptr;
+        const float* row32 = nullptr;
+        if (FROM_BF16) row16 = static_cast<const uint16_t*>(src) + (size_t)(perm[p] / top_k) * K;
+        else row32 = static_cast<const float*>(src) + (size_t)p * K;
 #pragma unroll
-    for (int u = 0; u < U; ++u) split_load8<FROM_BF16>(src, r, K, (c0 + 2 * u) * kChunkK + 8 * l16, vv[u]);
-    const SplitPlace at = split_places<FROM_BF16>(r, top_k, n_rows, inv, row_tile, tile_row0, lane);
-    const size_t block = act_block_bytes(TERMS, tile_tokens, false);
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const int c = c0 + 2 * u;
-        float (&v)[8] = vv[u];
-        uint2 bytes[TERMS];
-        uint32_t scales[TERMS];
-#pragma unroll
-        for (int t = 0; t < TERMS; ++t) {
-            const float amax = block_amax(v);
-            const int ef = (int)((__float_as_uint(amax) >> 23) & 0xffu);
-            const int sb = amax > 0.f ? max(ef - 7, 0) : 127;  // E8M0 byte: amax / scale in [128, 256)
-            const float inverse = __uint_as_float((uint32_t)(254 - sb) << 23);
-            const float scale = sb > 0 ? __uint_as_float((uint32_t)sb << 23) : __uint_as_float(0x00400000u);
-            __nv_fp8x2_storage_t q[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                q[i] = __nv_cvt_float2_to_fp8x2(make_float2(v[2 * i] * inverse, v[2 * i + 1] * inverse), __NV_SATFINITE, __NV_E4M3);
-            bytes[t] = make_uint2((uint32_t)q[0] | ((uint32_t)q[1] << 16), (uint32_t)q[2] | ((uint32_t)q[3] << 16));
-            if (t + 1 < TERMS) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const __half2_raw back = __nv_cvt_fp8x2_to_halfraw2(q[i], __NV_E4M3);
-                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&back));
-                    v[2 * i] -= f.x * scale;
-                    v[2 * i + 1] -= f.y * scale;
+        for (int u = 0; u < U; ++u) {
+            const int k0 = (c0 + u) * kChunkK + 4 * lane;
+            vv[u][0] = vv[u][1] = vv[u][2] = vv[u][3] = 0.f;
+            if (c0 + u < n_chunks && k0 < K) {
+                if (FROM_BF16) {
+                    const uint2 raw = *reinterpret_cast<const uint2*>(row16 + k0);
+                    vv[u][0] = __uint_as_float(raw.x << 16);
+                    vv[u][1] = __uint_as_float(raw.x & 0xffff0000u);
+                    vv[u][2] = __uint_as_float(raw.y << 16);
+                    vv[u][3] = __uint_as_float(raw.y & 0xffff0000u);
+                } else {
+                    const float4 raw = *reinterpret_cast<const float4*>(row32 + k0);
+                    vv[u][0] = raw.x; vv[u][1] = raw.y; vv[u][2] = raw.z; vv[u][3] = raw.w;
                 }
             }
-            scales[t] = chunk_scales((uint32_t)sb, lane);
         }
-        for (int s = 0; s < (FROM_BF16 ? top_k : 1); ++s) {
-            const int tile = __shfl_sync(0xffffffffu, at.tile, s), n = __shfl_sync(0xffffffffu, at.row, s);
-            if (c >= n_chunks || n < 0) continue;
-            uint8_t* blk = act + ((size_t)tile * n_chunks + c) * block;
-            uint8_t* row = blk + act_header_bytes(TERMS) + (size_t)(n >> 3) * TERMS * 1024 + (n & 7) * 128 + (((l16 >> 1) ^ (n & 7)) << 4) + ((l16 & 1) << 3);
+    }
+    const int tile = row_tile[p], j = p - tile_row0[tile];
+    const int npad = (tile_rows[tile] + 7) & ~7;
 #pragma unroll
-            for (int t = 0; t < TERMS; ++t) {
-                *reinterpret_cast<uint2*>(row + t * 1024) = bytes[t];
-                if (l16 == 0) *reinterpret_cast<uint32_t*>(blk + t * 512 + (n & 31) * 16 + (n >> 5) * 4) = scales[t];
+    for (int u = 0; u < U; ++u) {
+        const int c = c0 + u;
+        if (c >= n_chunks) break;
+        float* v = vv[u];
+        uint8_t* blk = act + ((size_t)tile * n_chunks + c) * act_block_bytes(TERMS, tile_tokens, STACK);
+#pragma unroll
+        for (int t = 0; t < TERMS; ++t) {
+            float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+            int ef = (int)((__float_as_uint(amax) >> 23) & 0xffu);
+            int sb = amax > 0.f ? max(ef - 7, 0) : 127;           // E8M0 byte: amax / scale in [128, 256)
+            float inv = __uint_as_float((uint32_t)(254 - sb) << 23);
+            float scale = sb > 0 ? __uint_as_float((uint32_t)sb << 23) : __uint_as_float(0x00400000u);
+            __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[0] * inv, v[1] * inv), __NV_SATFINITE, __NV_E4M3);
+            __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[2] * inv, v[3] * inv), __NV_SATFINITE, __NV_E4M3);
+            // row of this term inside the block and the place of its scale word
+            const int n = STACK ? t * npad + j : j;
+            uint8_t* row_ptr = STACK ? blk + 1024 + (size_t)(n >> 3) * 1024
+                                     : blk + act_header_bytes(TERMS) + ((size_t)(n >> 3) * TERMS + t) * 1024;
+            *reinterpret_cast<uint32_t*>(row_ptr + (n & 7) * 128 + (((lane >> 2) ^ (n & 7)) << 4) + ((lane & 3) << 2)) =
+                (uint32_t)lo | ((uint32_t)hi << 16);
+            if (t + 1 < TERMS) {
+                __half2_raw blo = __nv_cvt_fp8x2_to_halfraw2(lo, __NV_E4M3), bhi = __nv_cvt_fp8x2_to_halfraw2(hi, __NV_E4M3);
+                float2 flo = __half22float2(*reinterpret_cast<__half2*>(&blo)), fhi = __half22float2(*reinterpret_cast<__half2*>(&bhi));
+                v[0] -= flo.x * scale; v[1] -= flo.y * scale; v[2] -= fhi.x * scale; v[3] -= fhi.y * scale;
             }
+            uint32_t w = (uint32_t)sb;
+            w |= __shfl_sync(0xffffffffu, (uint32_t)sb, 8) << 8;
+            w |= __shfl_sync(0xffffffffu, (uint32_t)sb, 16) << 16;
+            w |= __shfl_sync(0xffffffffu, (uint32_t)sb, 24) << 24;
+            if (lane == 0) *reinterpret_cast<uint32_t*>(blk + (STACK ? 0 : t * 512) + (n & 31) * 16 + (n >> 5) * 4) = w;
         }
     }
 }
@@ -788,49 +740,56 @@ __global__ void __launch_bounds__(256) split_rows_fp4_kernel(const void* __restr
 
 // MXFP4 quantisation of activation rows for tcgen05.mma.kind::mxf4 at prefill (both operands 4-bit):
 // per block of 32 along K the E8M0 scale is 2^(floor(log2 amax) - 2), so amax lands in [4, 8) and
-// clips to 6; every value is rounded to the nearest e2m1 magnitude, ties to the even code.  Work split as
-// in split_rows_kernel.  Block per (token tile, chunk):
+// clips to 6; every value is rounded to the nearest e2m1 magnitude, ties to the even code.  One warp
+// per (sorted row p, 128-wide chunk), lane l owns 4 elements.  Block per (token tile, chunk):
 // [512 B scale atom: byte (n % 32) * 16 + (n / 32) * 4 + kb for tile row n, k-block kb]
 // [16 row groups x 512 B: rows of 64 bytes (128 codes, low nibble = even column) in the
 // 64-byte-swizzled K-major layout, 16-byte unit u of row n at u ^ ((n >> 1) & 3)].
 constexpr int kQuant4BlockBytes = 512 + 128 * 64;
 
 template <bool FROM_BF16>
-__global__ void __launch_bounds__(256) quant_rows_mxfp4_kernel(const void* __restrict__ src, const int32_t* __restrict__ inv, int top_k, int K,
-                                                               int n_src, int n_rows, const int32_t* __restrict__ row_tile,
+__global__ void __launch_bounds__(256) quant_rows_mxfp4_kernel(const void* __restrict__ src, const int32_t* __restrict__ perm,
+                                                               int top_k, int K, int n_rows, const int32_t* __restrict__ row_tile,
                                                                const int32_t* __restrict__ tile_row0, uint8_t* __restrict__ act) {
     pdl_launch_dependents();
     pdl_wait();
-    constexpr int U = kSplitChunksPerWarp / 2;
-    const int n_chunks = round_up_int(K, kChunkK) / kChunkK, groups = (n_chunks + 2 * U - 1) / (2 * U);
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, l16 = lane & 15;
-    if (warp >= n_src * groups) return;
-    const int r = warp / groups, c0 = (warp % groups) * 2 * U + (lane >> 4);  // this lane's first chunk
-    float vv[U][8];
-#pragma unroll
-    for (int u = 0; u < U; ++u) split_load8<FROM_BF16>(src, r, K, (c0 + 2 * u) * kChunkK + 8 * l16, vv[u]);
-    const SplitPlace at = split_places<FROM_BF16>(r, top_k, n_rows, inv, row_tile, tile_row0, lane);
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const int c = c0 + 2 * u;
-        const float (&v)[8] = vv[u];
-        const float amax = block_amax(v);
-        const int ef = (int)((__float_as_uint(amax) >> 23) & 0xffu);
-        const int sb = amax > 0.f ? min(max(ef - 2, 1), 254) : 127;             // E8M0 byte of the block scale
-        const float inverse = __uint_as_float((uint32_t)(254 - sb) << 23);       // 1 / scale, exact
-        uint32_t codes = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            codes |= (uint32_t)__nv_cvt_float2_to_fp4x2(make_float2(v[2 * i] * inverse, v[2 * i + 1] * inverse), __NV_E2M1, cudaRoundNearest) << (8 * i);
-        const uint32_t scales = chunk_scales((uint32_t)sb, lane);
-        for (int s = 0; s < (FROM_BF16 ? top_k : 1); ++s) {
-            const int tile = __shfl_sync(0xffffffffu, at.tile, s), n = __shfl_sync(0xffffffffu, at.row, s);
-            if (c >= n_chunks || n < 0) continue;
-            uint8_t* blk = act + ((size_t)tile * n_chunks + c) * kQuant4BlockBytes;
-            *reinterpret_cast<uint32_t*>(blk + 512 + (size_t)(n >> 3) * 512 + (n & 7) * 64 + (((l16 >> 2) ^ ((n >> 1) & 3)) << 4) + ((l16 & 3) << 2)) = codes;
-            if (l16 == 0) *reinterpret_cast<uint32_t*>(blk + (n & 31) * 16 + (n >> 5) * 4) = scales;
+    const int Kp = round_up_int(K, kChunkK), n_chunks = Kp / kChunkK;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (warp >= n_rows * n_chunks) return;
+    const int p = warp / n_chunks, c = warp - p * n_chunks;
+    const int src_row = FROM_BF16 ? perm[p] / top_k : p;
+    const int k0 = c * kChunkK + 4 * lane;
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (k0 < K) {
+        if (FROM_BF16) {
+            const uint2 raw = *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(src) + (size_t)src_row * K + k0);
+            v[0] = __uint_as_float(raw.x << 16);
+            v[1] = __uint_as_float(raw.x & 0xffff0000u);
+            v[2] = __uint_as_float(raw.y << 16);
+            v[3] = __uint_as_float(raw.y & 0xffff0000u);
+        } else {
+            const float4 raw = *reinterpret_cast<const float4*>(static_cast<const float*>(src) + (size_t)src_row * K + k0);
+            v[0] = raw.x; v[1] = raw.y; v[2] = raw.z; v[3] = raw.w;
         }
     }
+    float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+    const int ef = (int)((__float_as_uint(amax) >> 23) & 0xffu);
+    const int sb = amax > 0.f ? min(max(ef - 2, 1), 254) : 127;       // E8M0 byte of the block scale
+    const float inv = __uint_as_float((uint32_t)(254 - sb) << 23);     // 1 / scale, exact
+    const __nv_fp4x2_storage_t lo = __nv_cvt_float2_to_fp4x2(make_float2(v[0] * inv, v[1] * inv), __NV_E2M1, cudaRoundNearest);
+    const __nv_fp4x2_storage_t hi = __nv_cvt_float2_to_fp4x2(make_float2(v[2] * inv, v[3] * inv), __NV_E2M1, cudaRoundNearest);
+    const int tile = row_tile[p], n = p - tile_row0[tile];
+    uint8_t* blk = act + ((size_t)tile * n_chunks + c) * kQuant4BlockBytes;
+    *reinterpret_cast<uint16_t*>(blk + 512 + (size_t)(n >> 3) * 512 + (n & 7) * 64 + (((lane >> 3) ^ ((n >> 1) & 3)) << 4) +
+                                 ((lane & 7) << 1)) = (uint16_t)((uint32_t)lo | ((uint32_t)hi << 8));
+    uint32_t w = (uint32_t)sb;
+    w |= __shfl_sync(0xffffffffu, (uint32_t)sb, 8) << 8;
+    w |= __shfl_sync(0xffffffffu, (uint32_t)sb, 16) << 16;
+    w |= __shfl_sync(0xffffffffu, (uint32_t)sb, 24) << 24;
+    if (lane == 0) *reinterpret_cast<uint32_t*>(blk + (n & 31) * 16 + (n >> 5) * 4) = w;
 }
 
 // ---------------------------------------------------------------------------------------

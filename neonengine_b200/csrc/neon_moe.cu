@@ -559,10 +559,8 @@ template <int TERMS, bool FROM_BF16>
 void launch_split(neon_moe_handle* h, int tile_tokens, const TileList& tl, const void* src, int K, int n, int top_k,
                   const float* amax, float amax_const, uint8_t* act, float* row_scale, cudaStream_t st) {
     const int n_chunks = round_up_int(K, kChunkK) / kChunkK;
-    const int n_src = FROM_BF16 ? n / top_k : n;  // tokens, or sorted rows
-    const dim3 prefill_grid((n_src * ((n_chunks + kSplitChunksPerWarp - 1) / kSplitChunksPerWarp) + 7) / 8);
     if (tile_tokens > 32 && h->mxf4_prefill)
-        launch_k(h->pdl != 0, quant_rows_mxfp4_kernel<FROM_BF16>, prefill_grid, dim3(256), 0, st, src, (const int32_t*)h->inv, top_k, K, n_src, n,
+        launch_k(h->pdl != 0, quant_rows_mxfp4_kernel<FROM_BF16>, dim3((n * n_chunks + 7) / 8), dim3(256), 0, st, src, h->perm, top_k, K, n,
                  tl.row_tile, tl.row0, act);
     else if (tile_tokens <= 32 && h->mx4)
         launch_k(h->pdl != 0, split_rows_fp4_kernel<kMx4Terms, FROM_BF16>, dim3((n * n_chunks + 7) / 8), dim3(256), 0, st, src,
@@ -571,8 +569,9 @@ void launch_split(neon_moe_handle* h, int tile_tokens, const TileList& tl, const
         launch_k(h->pdl != 0, split_rows_stacked_kernel<TERMS, FROM_BF16>, dim3((n * n_chunks + 7) / 8), dim3(256), 0, st, src,
                  h->perm, top_k, K, n, tl.row_tile, tl.row0, tl.rows, tile_tokens, amax, amax_const, act, row_scale);
     else
-        launch_k(h->pdl != 0, split_rows_kernel<TERMS, FROM_BF16>, prefill_grid, dim3(256), 0, st, src, (const int32_t*)h->inv, top_k, K, n_src, n,
-                 tl.row_tile, tl.row0, tile_tokens, act);
+        launch_k(h->pdl != 0, split_rows_kernel<TERMS, FROM_BF16, false>,
+                 dim3((n * ((n_chunks + kSplitChunksPerWarp - 1) / kSplitChunksPerWarp) + 7) / 8), dim3(256), 0, st, src,
+                 h->perm, top_k, K, n, tl.row_tile, tl.row0, tl.rows, tile_tokens, act);
     h->launches++;
 }
 
