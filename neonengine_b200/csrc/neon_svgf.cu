@@ -549,26 +549,23 @@ int neon_svgf_set_history(neon_svgf_handle* h, const uint16_t* colour_a, const u
                           int ping_pong, int on_device) {
     if (!h) return NEON_MOE_EINVAL;
     SCU(h, cudaSetDevice(h->cfg.device));
-    if (h->last_stream) SCU(h, cudaStreamSynchronize(h->last_stream));
+    SCU(h, cudaStreamSynchronize(h->last_stream));  // also the NULL stream
     const size_t px = (size_t)h->cfg.width * h->cfg.height;
     const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     if (colour_a) SCU(h, cudaMemcpy(h->colour_a, colour_a, px * 8, kind)); else SCU(h, cudaMemset(h->colour_a, 0, px * 8));
     if (colour_b) SCU(h, cudaMemcpy(h->colour_b, colour_b, px * 8, kind)); else SCU(h, cudaMemset(h->colour_b, 0, px * 8));
     h->cur_a = 0;
     if (moments) {
-        float4* tmp = nullptr;
-        SCU(h, cudaMalloc(&tmp, px * 16));
-        cudaError_t e = cudaMemcpy(tmp, moments, px * 16, kind);
-        if (e == cudaSuccess) {
-            k_split_moments<<<(unsigned)((px + 255) / 256), 256, 0, h->own_stream>>>(px, tmp, h->mom_a[0], h->mom_b[0]);
-            e = cudaStreamSynchronize(h->own_stream);
-        }
-        cudaFree(tmp);
-        if (e != cudaSuccess) return sfail(h, NEON_MOE_ECUDA, "loading the moments failed: %s", cudaGetErrorString(e));
+        // through the guide image, which every frame writes before it reads it, and on the copy's own stream: a
+        // device-to-device or pageable copy may still be under way when its call returns
+        SCU(h, cudaMemcpy(h->guide, moments, px * 16, kind));
+        k_split_moments<<<(unsigned)((px + 255) / 256), 256, 0, nullptr>>>(px, h->guide, h->mom_a[0], h->mom_b[0]);
+        SCU(h, cudaGetLastError());
     } else {
         SCU(h, cudaMemset(h->mom_a[0], 0, px * 8));
         SCU(h, cudaMemset(h->mom_b[0], 0, px * 8));
     }
+    SCU(h, cudaStreamSynchronize(nullptr));  // the next frame may run on a stream that the NULL stream does not order
     h->ping_pong = ping_pong != 0;
     return NEON_MOE_OK;
 }
