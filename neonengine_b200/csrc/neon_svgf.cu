@@ -25,6 +25,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <string>
 #include <vector>
@@ -358,18 +359,13 @@ __global__ void k_copy(size_t n, const uchar4* __restrict__ image, uint2* __rest
     dst[i] = pack_rgba16(c.x / 255.0f, c.y / 255.0f, c.z / 255.0f, c.w / 255.0f);
 }
 
-// ---- the moments image {history length, first moment, second moment, variance} <-> its two planes ----
+// ---- the moments image {history length, first moment, second moment, variance} -> its two planes ----
 __global__ void k_split_moments(size_t n, const float4* __restrict__ m, float2* __restrict__ a, float2* __restrict__ b) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 v = m[i];
     a[i] = make_float2(v.x, v.z);
     b[i] = make_float2(v.y, v.w);
-}
-__global__ void k_join_moments(size_t n, const float2* __restrict__ a, const float2* __restrict__ b, float4* __restrict__ m) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    m[i] = make_float4(a[i].x, b[i].x, a[i].y, b[i].y);
 }
 
 thread_local std::string g_svgf_create_error;
@@ -650,7 +646,7 @@ int neon_svgf_denoise_host(neon_svgf_handle* h, const float* position, const flo
 int neon_svgf_read(neon_svgf_handle* h, const char* name, void* dst, uint64_t bytes) {
     if (!h || !name || !dst) return NEON_MOE_EINVAL;
     SCU(h, cudaSetDevice(h->cfg.device));
-    if (h->last_stream) SCU(h, cudaStreamSynchronize(h->last_stream));
+    SCU(h, cudaStreamSynchronize(h->last_stream));  // also the NULL stream
     const size_t px = (size_t)h->cfg.width * h->cfg.height;
     const void* src = nullptr;
     size_t need = 0;
@@ -664,14 +660,16 @@ int neon_svgf_read(neon_svgf_handle* h, const char* name, void* dst, uint64_t by
         return NEON_MOE_OK;
     } else return sfail(h, NEON_MOE_EINVAL, "unknown buffer '%s'", name);
     if (bytes != need) return sfail(h, NEON_MOE_EINVAL, "%s is %zu bytes, not %llu", name, need, (unsigned long long)bytes);
-    if (!src) {  // the moments: joined from their planes
-        float4* tmp = nullptr;
-        SCU(h, cudaMalloc(&tmp, px * 16));
-        k_join_moments<<<(unsigned)((px + 255) / 256), 256, 0, h->own_stream>>>(px, h->mom_a[h->cur_a], h->mom_b[0], tmp);
-        cudaError_t e = cudaStreamSynchronize(h->own_stream);
-        if (e == cudaSuccess) e = cudaMemcpy(dst, tmp, need, cudaMemcpyDeviceToHost);
-        cudaFree(tmp);
-        if (e != cudaSuccess) return sfail(h, NEON_MOE_ECUDA, "reading the moments failed: %s", cudaGetErrorString(e));
+    if (!src) {  // the moments: joined from their planes on the host
+        std::unique_ptr<float[]> planes(new (std::nothrow) float[4 * px]);
+        if (!planes) return sfail(h, NEON_MOE_ECUDA, "out of host memory");
+        const float *a = planes.get(), *b = a + 2 * px;
+        SCU(h, cudaMemcpy(planes.get(), h->mom_a[h->cur_a], px * 8, cudaMemcpyDeviceToHost));
+        SCU(h, cudaMemcpy(planes.get() + 2 * px, h->mom_b[0], px * 8, cudaMemcpyDeviceToHost));
+        for (size_t i = 0; i < px; ++i) {
+            const float m[4] = {a[2 * i], b[2 * i], a[2 * i + 1], b[2 * i + 1]};
+            memcpy(static_cast<char*>(dst) + 16 * i, m, 16);
+        }
         return NEON_MOE_OK;
     }
     SCU(h, cudaMemcpy(dst, src, need, cudaMemcpyDeviceToHost));

@@ -1,4 +1,5 @@
-"""GPU checks of the denoiser's state between frames: history loaded from device and from pageable host memory.
+"""GPU checks of the denoiser's state between frames: history loaded from device and from pageable host memory, the
+moments read straight after a frame on the NULL stream.
 Bit-exact against the restatement."""
 import ctypes
 
@@ -52,4 +53,23 @@ def test_frame_from_device_history():
     torch.cuda.synchronize()
     np.testing.assert_array_equal(dimg.cpu().numpy(), image)
     _check_state(dn, st)
+    dn.close()
+
+
+def test_moments_straight_after_a_frame():
+    import torch
+    w, h = 1920, 1080
+    dn = _denoiser(w, h)
+    frames = [svgf_synth.make_frame(w, h, i) for i in range(2)]
+    dg = [[torch.from_numpy(a).cuda() for a in g] for g, _ in frames]
+    dimg = [torch.from_numpy(image).cuda() for _, image in frames]
+    torch.cuda.synchronize()
+    for g, image in zip(dg, dimg):
+        dn.render(g, image)  # the NULL stream; nothing waits for it before the read
+    got = _read(dn, "moments", np.empty((h, w, 4), np.float32))
+    np.testing.assert_array_equal(_read(dn, "moments", got), got)
+    st = svgf.State.zeros(w, h)
+    for g, image in frames:
+        svgf.frame(g, image, st, 3, serial=False)
+    np.testing.assert_array_equal(got, st.data)
     dn.close()
