@@ -65,7 +65,9 @@ int neon_svgf_set_history(neon_svgf_handle* h, const uint16_t* colour_a, const u
 /* One frame, enqueued on cuda_stream.  Device pointers: position, normal (w = mesh id),
  * barycentric, motion: rgba32f, read only; image: rgba8, the path tracer's output on entry, the
  * denoised frame on return.  The launch sequence of a given argument set is captured into a CUDA
- * graph the first time and replayed afterwards (option use_graphs). */
+ * graph the first time and replayed afterwards (option use_graphs).  A frame enqueued while the
+ * caller captures cuda_stream becomes part of the caller's graph: each replay is one more frame of the
+ * moments' history, with the ping-pong flag (which history image is which) as it was at the capture. */
 int neon_svgf_denoise(neon_svgf_handle* h, const float* position, const float* normal, const float* barycentric,
                       const float* motion, uint8_t* image, void* cuda_stream);
 

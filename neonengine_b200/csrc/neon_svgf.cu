@@ -381,6 +381,7 @@ struct neon_svgf_handle {
     float4* guide = nullptr;                         // {normal, depth} of the frame being filtered
     uint8_t* surface = nullptr;                      // whether its pixels show a surface
     int ping_pong = 0, cur_a = 0;
+    bool settle = false;  // a caller has captured frames, whose graphs name the buffers: every frame leaves the state in mom_a[cur_a]
     float4* stage[4] = {nullptr, nullptr, nullptr, nullptr};  // device copies of host G-buffers (denoise_host)
     uchar4* stage_image = nullptr;
     int64_t launches = 0;
@@ -390,6 +391,7 @@ struct neon_svgf_handle {
     struct Cached {
         Frame fr;
         int ping_pong, cur_a;
+        bool settle;
         cudaGraphExec_t exec;
     };
     std::vector<Cached> graphs;
@@ -443,7 +445,8 @@ bool allow_tile() {
 }
 
 // the kernels of one frame in the reference's dispatch order; ev (optional) gets 3 event marks.
-// ping_pong is the flag's value BEFORE the frame (RayTracingRast::renderCompute flips it), cur_a that of h->cur_a.
+// ping_pong is the flag's value BEFORE the frame (RayTracingRast::renderCompute flips it), cur_a that of h->cur_a; the
+// frame leaves the state in mom_a[cur_a ^ 1], with h->settle in mom_a[cur_a].
 int record_frame(neon_svgf_handle* h, const Frame& fr, int ping_pong, int cur_a, cudaStream_t st, cudaEvent_t* ev = nullptr) {
     const int w = h->cfg.width, ht = h->cfg.height, iters = h->cfg.atrous_iterations;
     const dim3 grid((w + kBlockX - 1) / kBlockX, (ht + kBlockY - 1) / kBlockY), block(kBlockX, kBlockY);
@@ -477,6 +480,8 @@ int record_frame(neon_svgf_handle* h, const Frame& fr, int ping_pong, int cur_a,
         const size_t px = (size_t)w * ht;
         k_copy<<<(unsigned)((px + 255) / 256), 256, 0, st>>>(px, fr.image, prev); ++n;
     }
+    if (h->settle && cudaMemcpyAsync(h->mom_a[cur_a], h->mom_a[cur_a ^ 1], (size_t)w * ht * sizeof(float2), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+        return -1;
     if (ev) cudaEventRecord(ev[2], st);
     h->launches_per_frame = n;
     return cudaGetLastError() == cudaSuccess ? n : -1;
@@ -550,15 +555,14 @@ int neon_svgf_set_history(neon_svgf_handle* h, const uint16_t* colour_a, const u
     const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     if (colour_a) SCU(h, cudaMemcpy(h->colour_a, colour_a, px * 8, kind)); else SCU(h, cudaMemset(h->colour_a, 0, px * 8));
     if (colour_b) SCU(h, cudaMemcpy(h->colour_b, colour_b, px * 8, kind)); else SCU(h, cudaMemset(h->colour_b, 0, px * 8));
-    h->cur_a = 0;
     if (moments) {
         // through the guide image, which every frame writes before it reads it, and on the copy's own stream: a
         // device-to-device or pageable copy may still be under way when its call returns
         SCU(h, cudaMemcpy(h->guide, moments, px * 16, kind));
-        k_split_moments<<<(unsigned)((px + 255) / 256), 256, 0, nullptr>>>(px, h->guide, h->mom_a[0], h->mom_b[0]);
+        k_split_moments<<<(unsigned)((px + 255) / 256), 256, 0, nullptr>>>(px, h->guide, h->mom_a[h->cur_a], h->mom_b[0]);
         SCU(h, cudaGetLastError());
     } else {
-        SCU(h, cudaMemset(h->mom_a[0], 0, px * 8));
+        SCU(h, cudaMemset(h->mom_a[h->cur_a], 0, px * 8));
         SCU(h, cudaMemset(h->mom_b[0], 0, px * 8));
     }
     SCU(h, cudaStreamSynchronize(nullptr));  // the next frame may run on a stream that the NULL stream does not order
@@ -578,14 +582,15 @@ int neon_svgf_denoise(neon_svgf_handle* h, const float* position, const float* n
     const int pp = h->ping_pong, ca = h->cur_a;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     bool graphs = h->use_graphs != 0;
-    if (graphs && (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)) {
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         graphs = false;  // inside the caller's own capture: record the kernels directly
+        if (cs != cudaStreamCaptureStatusNone) h->settle = true;
     }
     if (graphs) {
         neon_svgf_handle::Cached* hit = nullptr;
         for (auto& g : h->graphs)
-            if (g.ping_pong == pp && g.cur_a == ca && !memcmp(&g.fr, &fr, sizeof fr)) { hit = &g; break; }
+            if (g.ping_pong == pp && g.cur_a == ca && g.settle == h->settle && !memcmp(&g.fr, &fr, sizeof fr)) { hit = &g; break; }
         if (!hit) {
             if (h->graphs.size() >= 32) drop_graphs(h);
             SCU(h, cudaStreamBeginCapture(h->own_stream, cudaStreamCaptureModeThreadLocal));
@@ -600,7 +605,7 @@ int neon_svgf_denoise(neon_svgf_handle* h, const float* position, const float* n
                 h->use_graphs = 0;  // capture is not available here: stay eager
                 graphs = false;
             } else {
-                h->graphs.push_back({fr, pp, ca, exec});
+                h->graphs.push_back({fr, pp, ca, h->settle, exec});
                 hit = &h->graphs.back();
             }
         }
@@ -615,7 +620,7 @@ int neon_svgf_denoise(neon_svgf_handle* h, const float* position, const float* n
         h->launches += n;
     }
     h->ping_pong = !pp;
-    h->cur_a = ca ^ 1;
+    if (!h->settle) h->cur_a = ca ^ 1;
     h->last_stream = st;
     return NEON_MOE_OK;
 }
@@ -693,7 +698,7 @@ int neon_svgf_profile_frame(neon_svgf_handle* h, const float* position, const fl
     else {
         h->launches += n;
         h->ping_pong = !h->ping_pong;
-        h->cur_a ^= 1;
+        if (!h->settle) h->cur_a ^= 1;
         h->last_stream = st;
         for (int i = 0; i < 2; ++i) {
             float ms = 0.0f;

@@ -1,5 +1,5 @@
 """GPU checks of the denoiser's state between frames: history loaded from device and from pageable host memory, the
-moments read straight after a frame on the NULL stream.
+moments read straight after a frame on the NULL stream, frames that the caller captures and replays between others.
 Bit-exact against the restatement."""
 import ctypes
 
@@ -72,4 +72,56 @@ def test_moments_straight_after_a_frame():
     for g, image in frames:
         svgf.frame(g, image, st, 3, serial=False)
     np.testing.assert_array_equal(got, st.data)
+    dn.close()
+
+
+@pytest.mark.parametrize("before", [0, 1])
+@pytest.mark.parametrize("captured", [1, 2])
+def test_captured_frames_go_on_with_the_history(before, captured):
+    import torch
+    w, h = 96, 64
+    dn, st = _denoiser(w, h), svgf.State.zeros(w, h)
+    g, image = svgf_synth.make_frame(w, h, 1)
+    dg, fresh = [torch.from_numpy(a).cuda() for a in g], torch.from_numpy(image).cuda()
+    dimg = fresh.clone()
+
+    def eager():
+        dimg.copy_(fresh)
+        dn.render(dg, dimg)
+        check(1, st.ping_pong)
+
+    def check(frames, ping_pong):
+        st.ping_pong = ping_pong
+        for _ in range(frames):
+            want = image.copy()
+            svgf.frame(g, want, st, 3, serial=False)
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(dimg.cpu().numpy(), want)
+        np.testing.assert_array_equal(_read(dn, "moments", st.data), st.data)
+        np.testing.assert_array_equal(_read(dn, "colour_a", st.colour_a), st.colour_a)
+        np.testing.assert_array_equal(_read(dn, "colour_b", st.colour_b), st.colour_b)
+
+    for _ in range(before):
+        eager()
+    flag = st.ping_pong
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=side):
+        for _ in range(captured):
+            dimg.copy_(fresh)
+            dn.render(dg, dimg, stream=side)
+    st.ping_pong = (flag + captured) & 1  # what the captured calls left the handle's own flag at
+    for replays in (1, 2, 3):
+        for _ in range(replays):
+            own = st.ping_pong
+            graph.replay()
+            check(captured, flag)
+            st.ping_pong = own
+        eager()
+    history = _state(w, h)
+    torch.cuda.synchronize()
+    dn.set_history(history.colour_a, history.colour_b, history.data, flag)
+    st = history
+    graph.replay()
+    check(captured, flag)
     dn.close()
