@@ -1112,7 +1112,10 @@ static int launch_decode_sliced(neon_moe_handle* h, const void* hidden, int T, c
     return NEON_MOE_OK;
 }
 
-// A pass of one token as three kernels that stream weights (decode_stream.cuh).
+// A pass of one token as three kernels that stream weights (decode_stream.cuh).  Their f16 SwiGLU rows are scaled by a
+// bound of the values: g * sigmoid(alpha g) falls to -kSwishDepth / alpha for negative g, whatever the limit, which bounds
+// nothing useful for an alpha near zero and is no minimum for a negative one.
+constexpr float kSwishDepth = 0.27847f, kStreamMinAlpha = 1e-6f;
 static int launch_decode_stream(neon_moe_handle* h, const void* hidden, const float* logit_bias, float* out, cudaStream_t st) {
     const int H = h->cfg.hidden, I = h->cfg.inter, E = h->cfg.n_experts;
     StreamParams p{};
@@ -1121,8 +1124,9 @@ static int launch_decode_stream(neon_moe_handle* h, const void* hidden, const fl
     p.limit = h->cfg.swiglu_limit; p.alpha = h->cfg.swiglu_alpha;
     p.gu_w = h->gu_wt; p.gu_sfa = h->gu_sfa; p.dn_w = h->dn_wt; p.dn_sfa = h->dn_sfa; p.gu_bias = h->gu_bias; p.dn_bias = h->dn_bias;
     p.n_slices = std::max(1, std::min(kStrSlicesMax, kStrCluster * (kStrRouteThreads / 32) / E));
-    {   // |SwiGLU| <= limit * (limit + 1), which goes to [2^14, 2^15); kept where the factor and its inverse are normal
-        const float bound = h->cfg.swiglu_limit * (h->cfg.swiglu_limit + 1.f);
+    {   // |SwiGLU| <= max(limit, depth of g * sigmoid(alpha g) below zero) * (limit + 1), which goes to [2^14, 2^15); kept
+        // where the factor and its inverse are normal
+        const float bound = std::max(h->cfg.swiglu_limit, kSwishDepth / h->cfg.swiglu_alpha) * (h->cfg.swiglu_limit + 1.f);
         uint32_t bits;
         memcpy(&bits, &bound, 4);
         bits = (uint32_t)std::min(std::max(268 - (int)((bits >> 23) & 0xffu), 1), 253) << 23;
@@ -1258,7 +1262,8 @@ static int forward_eager(neon_moe_handle* h, const void* hidden, int T, const fl
     const int k = h->cfg.top_k, n = T * k;
     const bool prof = h->profiling && h->events_used + 5 <= 5 * kMaxProfiledForwards;
     const bool small = h->path == 2 && h->decode_fused && !prof && h->tile_override == 0 && !h->mx4 && !h->fuse_dispatch;
-    const bool streamed = small && T == 1 && h->decode_stream && h->stream_ready && h->decode_fused_tokens <= 1;
+    const bool streamed = small && T == 1 && h->decode_stream && h->stream_ready && h->decode_fused_tokens <= 1 &&
+                          h->cfg.swiglu_alpha >= kStreamMinAlpha;
     const bool one_launch = small && !streamed && T <= std::min(h->decode_max_tokens, h->decode_fused_tokens);
     if (streamed || one_launch) {
         int rc = streamed ? launch_decode_stream(h, hidden, logit_bias, out, st)

@@ -47,3 +47,33 @@ def test_scales_over_a_wide_range_and_a_zero_token():
         out, idx, w = run_device(layer, x)
         assert errors(out, oracle.experts(x, idx, w, W))[1] < 4e-6 and np.isfinite(out).all()
     layer.close()
+
+
+@pytest.mark.parametrize("limit,alpha", [(0.02, 1.702), (0.05, 1.702), (0.3, 0.1), (7.0, 0.01), (0.5, 1e-4), (50.0, 1.702)])
+def test_swiglu_bounds(limit, alpha):
+    """The gate's negative lobe is 0.278 / alpha deep, with gates far enough out to meet it."""
+    shape = synth.MoeShape(hidden=192, inter=128, n_experts=8, top_k=2, swiglu_limit=limit, swiglu_alpha=alpha)
+    W = synth.make_weights(shape, 7)
+    x = synth.make_hidden(1, W, 8)
+    # gates of a few times 1.28 / alpha, where the lobe is deepest
+    W.gate_up_scales[:] = np.clip(W.gate_up_scales.astype(int) + int(np.round(np.log2(4.0 / alpha))), 1, 250)
+    layer = make_layer(shape, W, max_tokens=1)
+    layer.set_option("use_graphs", 0)
+    before = layer.launch_count
+    out, idx, w = run_device(layer, x)
+    assert layer.launch_count - before == 3
+    ref = oracle.experts(x, idx, w, W)
+    assert np.isfinite(out).all() and errors(out, ref)[1] < 4e-6
+    layer.close()
+
+
+@pytest.mark.parametrize("alpha", [0.0, -1.0])
+def test_gates_without_a_bound_keep_off_the_stream(alpha):
+    shape = synth.MoeShape(hidden=192, inter=128, n_experts=8, top_k=2, swiglu_alpha=alpha)
+    W = synth.make_weights(shape, 7)
+    layer = make_layer(shape, W, max_tokens=1)
+    layer.set_option("use_graphs", 0)
+    before = layer.launch_count
+    out, idx, w = run_device(layer, synth.make_hidden(1, W, 8))
+    assert layer.launch_count - before == 1 and np.isfinite(out).all()
+    layer.close()
