@@ -77,3 +77,33 @@ def test_gates_without_a_bound_keep_off_the_stream(alpha):
     out, idx, w = run_device(layer, synth.make_hidden(1, W, 8))
     assert layer.launch_count - before == 1 and np.isfinite(out).all()
     layer.close()
+
+
+@pytest.fixture(scope="module")
+def small_layer():
+    shape = synth.MoeShape(hidden=192, inter=320, n_experts=8, top_k=2)
+    W = synth.make_weights(shape, 9)
+    layer = make_layer(shape, W, max_tokens=8)
+    layer.set_option("use_graphs", 0)
+    yield layer, synth.make_hidden(1, W, 10)
+    layer.close()
+
+
+def _with(layer, x, **options):
+    """Output and number of launches of a pass with the options set, which go back to their defaults."""
+    defaults = {"decode_fused": 1, "decode_fused_tokens": 1, "decode_stream": 1, "decode_sliced": 0}
+    for k, v in options.items():
+        layer.set_option(k, v)
+    before = layer.launch_count
+    out = run_device(layer, x)[0]
+    for k in options:
+        layer.set_option(k, defaults[k])
+    return out, layer.launch_count - before
+
+
+def test_no_tokens_for_the_one_launch_kernel_means_the_general_path(small_layer):
+    layer, x = small_layer
+    general, launches = _with(layer, x, decode_fused=0)
+    out, n = _with(layer, x, decode_fused_tokens=0)
+    assert n == launches > 3
+    np.testing.assert_array_equal(out, general)
