@@ -244,7 +244,8 @@ int neon_moe_status(neon_moe_handle* h, int* device_status_word);
  * combine, no dispatch pass; its CTAs wait for one another with bounded waits (status word on a timeout).
  * "decode_stream" (default 1): a pass of one token runs as three kernels that stream its experts' weights (29.4 us
  * at the gpt-oss-20b shapes; one launch 36.2 us, the general path 37.9 us) unless "decode_fused_tokens" is above 1, which
- * asks for the one-launch kernel, or "decode_fused" or "decode_fused_tokens" is 0, which asks for the general path.
+ * asks for the one-launch kernel as "decode_sliced" and "decode_stall_test" do, or "decode_fused" or "decode_fused_tokens" is 0,
+ * which asks for the general path.
  * "decode_sliced" (default 0): 1 runs one-launch passes of up to 4 tokens on the variant that slices the layer by
  * intermediate channel (each CTA computes 128 channels of one expert through both products, one grid-wide
  * barrier, no partial sums between the products); measured no faster (T = 1: 36.3 vs 35.1-36.5 us).

@@ -107,3 +107,13 @@ def test_no_tokens_for_the_one_launch_kernel_means_the_general_path(small_layer)
     out, n = _with(layer, x, decode_fused_tokens=0)
     assert n == launches > 3
     np.testing.assert_array_equal(out, general)
+
+
+def test_the_sliced_variant_is_taken_when_asked_for(small_layer):
+    layer, x = small_layer
+    sliced, n = _with(layer, x, decode_sliced=1)
+    want, m = _with(layer, x, decode_sliced=1, decode_fused_tokens=8)
+    one_launch, k = _with(layer, x, decode_stream=0)
+    assert n == m == k == 1
+    np.testing.assert_array_equal(sliced, want)
+    assert (sliced != one_launch).any()  # another order of the sums: not the one-launch kernel under another name
