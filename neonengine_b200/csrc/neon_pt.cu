@@ -5,7 +5,6 @@
 #include "../../include/neon_pt.h"
 
 #include <cuda_runtime.h>
-#include <xmmintrin.h>
 
 #include <algorithm>
 #include <cmath>
@@ -382,13 +381,16 @@ __global__ void __launch_bounds__(64) pt_frame_kernel(Scene sc, Camera cam, int 
 constexpr int kLeaf = 4, kBins = 16, kSample = 512, kSahDepth = 20, kMaxDepthBvh = kStack - 4;
 constexpr float kNodeCost = 1.5f;  // one node visit in units of one triangle test
 
+typedef float F4 __attribute__((vector_size(16)));  // the host compiler's own vectors: no architecture's intrinsics
 struct Box {  // four lanes, three of them used; a NaN coordinate leaves a bound as it is
-    __m128 lo = _mm_set1_ps(INFINITY), hi = _mm_set1_ps(-INFINITY);
-    void add(const Box& b) { lo = _mm_min_ps(b.lo, lo); hi = _mm_max_ps(b.hi, hi); }
+    F4 lo = {INFINITY, INFINITY, INFINITY, INFINITY}, hi = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    void add(const Box& b) {
+        lo = b.lo < lo ? b.lo : lo;
+        hi = b.hi > hi ? b.hi : hi;
+    }
     float area() const {
-        alignas(16) float e[4];
-        _mm_store_ps(e, _mm_sub_ps(hi, lo));
-        return e[0] >= 0.f ? e[0] * e[1] + e[1] * e[2] + e[2] * e[0] : 0.f;  // nothing added yet: empty
+        const float x = hi[0] - lo[0], y = hi[1] - lo[1], z = hi[2] - lo[2];
+        return x >= 0.f ? x * y + y * z + z * x : 0.f;  // nothing added yet: empty
     }
 };
 
@@ -401,7 +403,7 @@ struct Builder {
     int max_depth = 0, n_nodes = 0;  // nodes in the usual sense: inner nodes and leaves
     Box bin_boxes[3][kBins];
 
-    float centroid(int t, int a) const { return reinterpret_cast<const float*>(&cen[t].lo)[a]; }
+    float centroid(int t, int a) const { return cen[t].lo[a]; }
     Box bounds(int first, int count) const {
         Box b;
         for (int i = first; i < first + count; ++i) b.add(tri[order[i]]);
@@ -412,9 +414,9 @@ struct Builder {
         if (count <= 1 || depth >= kMaxDepthBvh) return first;
         Box c;
         for (int i = first; i < first + count; ++i) c.add(cen[order[i]]);
-        alignas(16) float lo[4], hi[4];
-        _mm_store_ps(lo, c.lo);
-        _mm_store_ps(hi, c.hi);
+        float lo[4], hi[4];
+        memcpy(lo, &c.lo, sizeof lo);
+        memcpy(hi, &c.hi, sizeof hi);
         const int n_bins = std::min(kBins, std::max(4, count));
         float scale[3];
         for (int a = 0; a < 3; ++a) scale[a] = (float)n_bins / (hi[a] - lo[a]);
@@ -489,9 +491,9 @@ struct Builder {
             const Box b = bounds(f, n);
             const int ref = build(f, n, depth + 1, b);
             nodes[node].ref[c] = ref;
-            alignas(16) float lo[4], hi[4];
-            _mm_store_ps(lo, b.lo);
-            _mm_store_ps(hi, b.hi);
+            float lo[4], hi[4];
+            memcpy(lo, &b.lo, sizeof lo);
+            memcpy(hi, &b.hi, sizeof hi);
             for (int a = 0; a < 3; ++a) {  // padded: the slab test must never lose a hit that lies on a face
                 const float pad = 1e-5f * std::max(1.f, std::max(std::fabs(lo[a]), std::fabs(hi[a])));
                 float* side = a == 0 ? nodes[node].x : (a == 1 ? nodes[node].y : nodes[node].z);
@@ -577,14 +579,15 @@ int neon_pt_create(const neon_pt_config* cfg, const neon_pt_vertex* vertices, in
     b.cen.resize(n_tri);
     for (int t = 0; t < n_tri; ++t) {
         b.order[t] = t;
-        __m128 p[3];
+        Box p[3];
         for (int c = 0; c < 3; ++c) {
             const float* v = vertices[indices[3 * t + c]].pos;
-            p[c] = _mm_set_ps(0.f, v[2], v[1], v[0]);
-            b.tri[t].lo = c ? _mm_min_ps(p[c], b.tri[t].lo) : p[c];
-            b.tri[t].hi = c ? _mm_max_ps(p[c], b.tri[t].hi) : p[c];
+            p[c].lo = p[c].hi = F4{v[0], v[1], v[2], 0.f};
         }
-        b.cen[t].lo = b.cen[t].hi = _mm_mul_ps(_mm_add_ps(_mm_add_ps(p[0], p[1]), p[2]), _mm_set1_ps(1.f / 3.f));
+        b.tri[t] = p[0];
+        b.tri[t].add(p[1]);
+        b.tri[t].add(p[2]);
+        b.cen[t].lo = b.cen[t].hi = (p[0].lo + p[1].lo + p[2].lo) * (1.f / 3.f);
     }
     b.last.resize(n_tri);
     b.nodes.reserve(n_tri);
