@@ -232,9 +232,9 @@ int neon_moe_status(neon_moe_handle* h, int* device_status_word);
  * kernel under programmatic dependent launch, 0.1086 vs 0.1078 ms per 64-token pass).
  * "tile_tokens" (default 0 = by batch size: 16 up to 16 tokens, 32 up to 224, else 128): forces the
  * token-tile size of the grouped GEMMs (16 and 32 use the stacked-term kernels).
- * "router_wide_max" (default 224): passes of up to this many tokens run the router with one CTA per
- * token, which also produces the per-token maxima the 16/32-token tiles scale by; larger passes use
- * the router that shares each weight read between 8 tokens.  "graph_max_tokens" (default 64): the
+ * "router_wide_max" (default -1 = 224 where larger passes route on tensor cores, else 384): passes of up to this many
+ * tokens run the router with one CTA per token, which also produces the per-token maxima the 16/32-token tiles scale
+ * by; larger passes use the router that shares each weight read between 8 tokens.  "graph_max_tokens" (default 64): the
  * largest pass that is replayed from a captured graph (measured gain above 64 tokens: ~1 us).
  * "router_mma" (default 1): passes above router_wide_max tokens compute the router logits on tensor
  * cores (mma.sync, 16 to 64 tokens per CTA; 32 or 128 experts); 0 = the CUDA-core router that shares each

@@ -62,8 +62,12 @@ struct neon_moe_handle {
     int max_stages = 0, ctas_per_sm = 1;
     int pdl = 1;                  // programmatic dependent launch between the kernels of a pass
     int tile_override = 0;        // 0 = token-tile size chosen from the batch size; 16 / 32 / 128 force it
-    int router_wide_max = 224;    // passes up to this many tokens use the one-CTA-per-token router, which also yields the token
-                                  // maxima the stacked-term tiles need - which passes of up to 224 tokens run on
+    // Passes up to this many tokens use the one-CTA-per-token router, which also yields the token maxima the stacked-term tiles
+    // need - which passes of up to 224 tokens run on.  -1: 224 where the tensor-core router takes over (300 tokens, 32 experts:
+    // 184 -> 178 us a pass), else 384: against the token-blocked router, us a pass at 225 / 256 / 300 / 384 tokens, 16 experts
+    // 105 / 109 / 124 / 139 and 113 / 109 / 117 / 134, 64 experts 266 / 267 / 284 / 297 and 278 / 274 / 282 / 292, 256 experts
+    // 880 / 895 / 927 / 941 and 919 / 929 / 940 / 954.
+    int router_wide_max = -1;
     int graph_max_tokens = 64;    // passes up to this many tokens are replayed from a captured CUDA graph
     int router_mma = 1;           // larger passes route on tensor cores (32 or 128 experts); 0 = the token-blocked CUDA-core router
     int sync_debug = 0;           // synchronise and check after every kernel (slow; names the failing kernel)
@@ -1162,15 +1166,23 @@ static int launch_decode_stream(neon_moe_handle* h, const void* hidden, const fl
     return NEON_MOE_OK;
 }
 
+static bool router_on_tensor_cores(const neon_moe_handle* h) {
+    return h->router_mma && (h->cfg.n_experts == 32 || h->cfg.n_experts == 128) && h->cfg.hidden % 32 == 0;
+}
+static int router_wide_max(const neon_moe_handle* h) {
+    return h->router_wide_max >= 0 ? h->router_wide_max : (router_on_tensor_cores(h) ? 224 : 384);
+}
+
 static void launch_router(neon_moe_handle* h, const void* hidden, int T, const float* logit_bias, int32_t* idx, float* w,
                           float* tok_amax, cudaStream_t st) {
     const int H = h->cfg.hidden, E = h->cfg.n_experts, k = h->cfg.top_k;
-    if (h->path == 2 && T > h->router_wide_max && h->router_mma && (E == 32 || E == 128) && H % 32 == 0) {
+    const bool wide = T <= router_wide_max(h);
+    if (h->path == 2 && !wide && router_on_tensor_cores(h)) {
         // tensor-core router: no token maxima (128-token tiles scale per block); token tiles that leave the CTAs one wave
         if (T <= 16 * h->n_sms) launch_router_mma<1, 3>(h, hidden, T, logit_bias, idx, w, st);
         else if (T <= 32 * h->n_sms) launch_router_mma<2, 2>(h, hidden, T, logit_bias, idx, w, st);
         else launch_router_mma<4, 1>(h, hidden, T, logit_bias, idx, w, st);
-    } else if (h->path == 2 && T > h->router_wide_max) {  // token-blocked router: no token maxima either
+    } else if (h->path == 2 && !wide) {  // token-blocked router: no token maxima either
         const size_t smem = (size_t)8 * H * 2 + (size_t)8 * E * sizeof(float);
         static bool configured[kMaxDevicesAttr] = {};
         if (!configured[h->cfg.device]) {
@@ -1292,7 +1304,7 @@ static int forward_eager(neon_moe_handle* h, const void* hidden, int T, const fl
         launch_router(h, hidden, T, logit_bias, h->idx, h->route_w, h->x_amax, st);
     }
     // the token maxima come from the decode routers only (the token-blocked router does not produce them)
-    int rc = experts_core(h, hidden, T, k, h->idx, 0, h->route_w, (h->path == 2 && T <= h->router_wide_max) ? h->x_amax : nullptr, out, st, prof,
+    int rc = experts_core(h, hidden, T, k, h->idx, 0, h->route_w, (h->path == 2 && T <= router_wide_max(h)) ? h->x_amax : nullptr, out, st, prof,
                           fused);
     if (rc) return rc;
     if (topk_idx) CU(h, cudaMemcpyAsync(topk_idx, h->idx, (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
