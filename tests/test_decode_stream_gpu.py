@@ -28,11 +28,13 @@ def test_against_the_oracle(hidden, inter, experts, top_k, seed):
     # f32 sums of at most 2880 exact products (their rounding adds up like its square root, 54 * 2^-24) and 22-bit activations
     assert mean_rel < 4e-6, (max_abs, mean_rel)
     np.testing.assert_array_equal(run_device(layer, x, lb)[0], out)  # two runs, the same bits
-    for option, launches in (("decode_stream", 1), ("decode_fused", 6)):
+    for option in ("decode_stream", "decode_fused"):
         layer.set_option(option, 0)
         before = layer.launch_count
         assert_close(out, run_device(layer, x, lb)[0], "stream vs " + option + " 0")
-        assert layer.launch_count - before >= launches
+        launches = layer.launch_count - before
+        # the one-launch kernel (which takes no more experts than there are SMs), the general path: not the stream again
+        assert launches == 1 if option == "decode_stream" and experts <= 128 else launches >= 6
     layer.close()
 
 

@@ -28,3 +28,18 @@ def test_router_line(experts, line):
         assert other == wide + 1
         assert launches(x, -1) == (wide if T <= line else other)
     layer.close()
+
+
+@pytest.mark.parametrize("experts,waves", [(32, 32), (128, 16), (128, 32)])
+def test_large_router_tiles(experts, waves):
+    """Passes of more than 16 and 32 tokens per SM take 32 and 64 tokens a CTA: the last tile holds one token."""
+    import numpy as np
+    import torch
+    from test_moe_gpu import check_against_oracle
+    T = waves * torch.cuda.get_device_properties(0).multi_processor_count + 1
+    shape = synth.MoeShape(hidden=320, inter=64, n_experts=experts, top_k=4)
+    W = synth.make_weights(shape, 4)
+    layer = make_layer(shape, W, max_tokens=T)
+    x = synth.make_hidden(T, W, 6)
+    check_against_oracle(layer, W, x, tokens=np.unique(np.r_[0, np.arange(0, T, 97), T - 2, T - 1]).astype(np.int32), what="router tiles")
+    layer.close()
