@@ -61,3 +61,16 @@ def test_a_crowd_takes_no_walk_for_every_particle():
         ms.append(start.elapsed_time(end))
     sim.close()
     assert min(ms) < 20.0, ms  # a walk of the lists for every particle took 135 ms, sorting the particles in memory 23
+
+
+def test_a_crowd_beyond_the_list_ends_the_walk():
+    from neonengine_b200.water_physics import WaterPhysics
+    cfg = WaterConfig(particles_per_side=10, collision_substeps=1)
+    pos = _positions(cfg, 1000, 0.0, 1)
+    sim = WaterPhysics(cfg, pos)
+    ms = []
+    for _ in range(6):
+        sim.set_particles(pos)
+        ms.append(sim.profile_step()["separate"])
+    sim.close()
+    assert min(ms) < 0.12, ms  # walking lists of 1000 to their end took 0.22 ms, stopping when 128 are found 0.05
