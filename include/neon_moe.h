@@ -242,7 +242,7 @@ int neon_moe_status(neon_moe_handle* h, int* device_status_word);
  * "decode_fused" (default 1) / "decode_fused_tokens" (default 1, at most 8): passes of up to that many
  * tokens (and top_k * T <= 32) run as ONE cooperative kernel - router, both expert products, SwiGLU and
  * combine, no dispatch pass; its CTAs wait for one another with bounded waits (status word on a timeout).
- * "decode_stream" (default 1): a pass of one token runs as three kernels that stream its experts' weights (29.4 us
+ * "decode_stream" (default 1): a pass of one token runs as three kernels that stream its experts' weights (28 us
  * at the gpt-oss-20b shapes; one launch 36.2 us, the general path 37.9 us) unless "decode_fused_tokens" is above 1, which
  * asks for the one-launch kernel as "decode_sliced" and "decode_stall_test" do, or "decode_fused" or "decode_fused_tokens" is 0,
  * which asks for the general path.

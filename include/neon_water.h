@@ -89,13 +89,15 @@ int neon_water_read_grid(neon_water_handle* h, const char* name, void* dst, uint
  * (pass 5), pressure apply + grid->particles + integrate (passes 6-8)}. */
 int neon_water_profile_step(neon_water_handle* h, double* ms4, void* cuda_stream);
 
-/* Reads (and clears) the device status word: non-zero when the fused Jacobi kernel's bounded
+/* Reads (and clears) the device status word: non-zero when the cooperative pressure kernel's bounded
  * grid-barrier wait gave up (the step's result is then invalid).  Synchronises the last stream. */
 int neon_water_status(neon_water_handle* h, int* device_status_word);
 
-/* Options: "use_graphs" (default 1); "fused_jacobi" (default 1 where the device supports
- * cooperative launches and the grid has at most 2 cells per resident thread: all pressure
- * iterations in one cooperative kernel with a grid-wide barrier; 0 = one launch per iteration). */
+/* Options: "use_graphs" (default 1); "fused_jacobi" (default 1: all pressure iterations in one launch, as a
+ * thread-block cluster with the pressure field in shared memory where it fits - up to 16 CTAs of at most
+ * 12288 cells, each at least a layer of the grid -, else, where the device supports cooperative launches and the
+ * grid has at most 2 cells per resident thread, as one cooperative kernel with a grid-wide barrier; 0, and
+ * larger grids: one launch per iteration). */
 int neon_water_set_option(neon_water_handle* h, const char* name, int64_t value);
 
 int64_t neon_water_launch_count(const neon_water_handle* h);

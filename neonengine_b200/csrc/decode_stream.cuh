@@ -23,7 +23,7 @@
 // holds it exactly down to 2^-28 of the largest (and to 2^-39 of it absolutely).  The f32 SwiGLU outputs enter the down
 // product as two f16 terms (22 bits), in columns 0-3 and 4-7.  Sums are f32 throughout.
 //
-// Measured per pass at the 20b shape: 29.4 us, one launch 36.2, seven launches 37.9 (128 experts: 34.4, 40.3, 45.8).
+// Measured per pass at the 20b shape: 27.6 to 28.0 us, one launch 36.2, seven launches 37.9 (128 experts: 34.4, 40.3, 45.8).
 // From two tokens on the grouped GEMM wins (two: 49.9 here against 46.1; eight: 148 against 72): a step's 300
 // instructions are a chain that 20 warps per SM do not hide at more bytes per SM (ncu: 1.9 instructions per clock, 54 % of
 // the DRAM rate), so the rule is one token.

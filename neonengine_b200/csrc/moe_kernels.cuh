@@ -650,7 +650,7 @@ __device__ __forceinline__ void topk_warp(const float* lgt, int E, int k, int la
 // k lands in, so every 16-byte load feeds two mma's.  The router weights are re-read by every CTA (from L2), hence the
 // larger token tiles for larger passes: MT keeps the CTAs within one wave.  Logits differ from the other routers' in
 // summation order only (~1e-6).  With four warps and one window in flight it took 36 us at any size up to 4096 tokens (43 us
-// with 128 experts), and 300 tokens on the one-CTA-per-token router 20 us: a 300-token pass 183.6 -> 177.9 us.
+// with 128 experts), and 300 tokens on the one-CTA-per-token router 20 us: a 300-token pass 182.4 -> 177.5 us.
 constexpr int kRouterMmaWarps = 16;
 template <int MT, int U>
 __global__ void __launch_bounds__(kRouterMmaWarps * 32)

@@ -139,10 +139,10 @@ __device__ inline bool tri_hit(const float4 ta, const float4 tb, float e2z, V3 o
 constexpr int kStack = 48;
 
 // Closest hit in (tmin, tmax), ties to the lower primitive index; any_hit: stop at the first hit.
-// Nearest child first, so that a hit found early prunes what lies behind it.  Bound by the node and triangle loads that
-// a ray's visits chain (all from L1 and L2) and by the lanes of a warp that wait for its longest ray; the engine's frame
-// (800 x 600, 50 lights, 1.75 M rays) takes 380 us, with one box per node, children in storage order, median splits and
-// a division per triangle test it took 2170 us.  The slab distances are
+// Nearest child first, so that a hit found early prunes what lies behind it.  Bound by instruction issue (64 % of the slots;
+// loads hit L1 to 99 %) and by the lanes of a warp that wait for its longest ray; the engine's frame (800 x 600, 50
+// lights, 1.75 M rays) takes 380 to 425 us by scene, with one box per node, children in storage order, median splits
+// and a division per triangle test it took 2130 to 2190 us.  The slab distances are
 // b * inv - o * inv with fused multiply-adds; a direction component below 1e-18 is replaced by it, which keeps
 // the products finite.  Both only move a box face by a few units of rounding of the ray's origin, which the padding of
 // the boxes covers (like the rounding of b - o), and the boxes never decide more than which triangles are tested.
