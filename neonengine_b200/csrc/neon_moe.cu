@@ -1274,8 +1274,8 @@ static int forward_eager(neon_moe_handle* h, const void* hidden, int T, const fl
     const int k = h->cfg.top_k, n = T * k;
     const bool prof = h->profiling && h->events_used + 5 <= 5 * kMaxProfiledForwards;
     const bool small = h->path == 2 && h->decode_fused && !prof && h->tile_override == 0 && !h->mx4 && !h->fuse_dispatch;
-    const bool streamed = small && T == 1 && h->decode_stream && h->stream_ready && h->decode_fused_tokens == 1 && !h->decode_sliced && !h->decode_stall_test &&
-                          h->cfg.swiglu_alpha >= kStreamMinAlpha;
+    const bool streamed = small && T == 1 && h->decode_stream && h->stream_ready && h->decode_fused_tokens == 1 &&
+                          !h->decode_sliced && !h->decode_stall_test && h->cfg.swiglu_alpha >= kStreamMinAlpha;
     const bool one_launch = small && !streamed && T <= std::min(h->decode_max_tokens, h->decode_fused_tokens);
     if (streamed || one_launch) {
         int rc = streamed ? launch_decode_stream(h, hidden, logit_bias, out, st)

@@ -219,10 +219,10 @@ __global__ void __launch_bounds__(kBlockX* kBlockY) k_temporal(int w, int h, Fra
 // ---- a-trous filter pass (raytracing_atrous.comp:59-160, iteration < 98) -------------------------
 // One CTA filters a tile of 32 x 16 pixels from shared memory, where the tile and its halo of two steps on each side
 // lie with the image's edges already repeated; a thread filters two pixels eight rows apart, so that everything after
-// the differences of a tap is one packed instruction for both.  Bound by instruction issue (slots 68 to 73 % active, the multiply-add pipe 41 %; 25
-// taps of about 40 instructions); a 1080p frame with 3 passes takes 334 us against 562 us with one pixel a thread,
-// separate taps of 44 bytes through L1 and colours summed in every pass.  STEP 0: any step, taps from global memory (steps
-// beyond 8, whose halo no longer fits).
+// the differences of a tap is one packed instruction for both.  Bound by instruction issue (25 taps of about 40
+// instructions; issue slots 68 to 73 % active, the multiply-add pipe 41 %); a 1080p frame with 3 passes takes 332 us
+// against 558 us with one pixel a thread, separate taps of 44 bytes through L1 and colours summed in every pass.  STEP 0:
+// any step, taps from global memory (steps beyond 8, whose halo no longer fits).
 // LAST: also the colour sums, the storage image and (copy_to != nullptr) its conversion back to floats in that
 // history image (the shaders' separate copy dispatch, raytracing_atrous.comp:66-70).
 constexpr int kTileX = 32, kTileY = 16, kFilterThreads = 256;
